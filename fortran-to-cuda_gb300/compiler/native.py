@@ -319,8 +319,8 @@ def advection(grid: Grid, u, v, w, ut=None, vt=None, wt=None, scalars=(), scalar
 
     ``variant`` FACES is the face-sharing kernel (the strict, bit-exact product
     path); DIRECT is the straightforward per-point kernel kept as a cross-check;
-    FAST is the fast-fp kernel (FMA-contracted, factored; within 1e-12 of each
-    field's maximum).
+    FAST is the fast-fp kernel (factored, in 64-bit fixed point; within 1e-12 of
+    each field's maximum).
     """
     fields = Fields()
     fields.u, fields.v, fields.w = u, v, w

@@ -3,7 +3,7 @@
 The reference schedules every nest the same way: axis order by unit-stride
 locality, no tiling, 256-thread blocks (compiler/scheduling/planner.py:82-123,
 compiler/ir/plan.py:31). Here a batched step has two shape choices: the tile
-height (4, 8 or 16 rows of 32 points; one warp per row plus an edge warp, the
+height (4, 8 or 16 rows of 32 points; one warp per row, the
 fast-fp kernel for 4 and 16) for the whole persistent launch, and per instance
 the depth of the z-chunk an item of work covers: deep chunks amortise the
 per-chunk prologue (the bottom faces of the first level), shallow chunks and

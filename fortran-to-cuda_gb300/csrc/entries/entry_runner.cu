@@ -141,13 +141,11 @@ int faces_spec(AdvArgs &a, bool fast, fort_scope_kernel_v1 &k) {
         const int sms = current_sm_count();
         ty = kFastTY;
         a.kz = fast_chunk_depth(a.nx, a.ny, a.nz, kFastTY, sms);
-        // the build for three CTAs per SM when the launch has enough CTAs (as launch_fast chooses)
-        const long long ctas = (long long)((a.nx + kFastTX - 1) / kFastTX) * ((a.ny + kFastTY - 1) / kFastTY) *
-                               ((a.nz + a.kz - 1) / a.kz);
-        k.function = ctas >= (long long)kFastDeepCtas * (sms > 0 ? sms : 152)
-                         ? (const void *)advection_fast_kernel<NS, MASK, kFastTY, kFastDeepCtasPerSM>
-                         : (const void *)advection_fast_kernel<NS, MASK, kFastTY>;
-        k.shared_bytes = 0;
+        k.function = (const void *)advection_fast_kernel<NS, MASK, kFastTY>;
+        k.shared_bytes = FastSmem<NS, kFastTY>::bytes;
+        static std::atomic<unsigned long long> configured{0};
+        if (configure_shared_once(configured, k.function, (int)k.shared_bytes) != cudaSuccess)
+            return fort_scope_report_error(FORT_SCOPE_RESOURCE, "cannot configure the fast-fp kernel");
     } else {
         using Smem = FaceSmem<NS, MASK>;
         static std::atomic<unsigned long long> configured{0};
@@ -162,7 +160,7 @@ int faces_spec(AdvArgs &a, bool fast, fort_scope_kernel_v1 &k) {
     k.grid[1] = (a.ny + ty - 1) / ty;
     k.grid[2] = (a.nz + a.kz - 1) / a.kz;
     k.block[0] = kFaceTX;
-    k.block[1] = ty + 1;
+    k.block[1] = fast ? ty : ty + 1;
     k.block[2] = 1;
     return FORT_SCOPE_OK;
 }

@@ -1,303 +1,383 @@
 // Factored ("fast-fp") z-marching advection kernel for sm_103a.
 //
 // The reference's --fast-fp build (compiler/resident/build.py:22,66-67) trades
-// the strict contract for FMA contraction. This kernel goes further in the same
-// direction: it evaluates the same tendencies as the strict face-sharing kernel
-// (advection_faces.cuh) through an algebraically regrouped form that spends
-// about 80 floating-point operations per grid point (U, V, W and three
-// scalars) where the reference grouping needs 126. GB300 issues FP64 at about
-// two lane operations per clock per SM, so the FP64 instruction count is what
-// bounds the step; everything else here (loads, shuffles, shared memory,
-// integer work) runs on otherwise idle pipes. That includes the twelve plain
-// products, which are computed on the integer pipes (pmul, soft_fp64.cuh; the
-// same correctly rounded values), leaving 68 instructions per point on the
-// FP64 pipe.
+// the strict contract for FMA contraction. This kernel computes the same
+// tendencies as the strict face-sharing kernel (advection_faces.cuh) through an
+// algebraically regrouped form, on the integer pipes. GB300 issues FP64 at 1.68
+// lane operations per clock per SM, 64-bit integer additions and 32 x 32 + 64
+// multiplications at 64 each, so what costs a thread one FP64 operation pays for
+// some forty integer ones: sums and products of a point's stencil are taken in
+// 64-bit fixed point at the point's own scale (wide_int.cuh), and FP64 converts
+// and scales each result, two operations per field instead of some twenty.
 //
 // Regrouping (exact in real arithmetic; A = 0.25/d per direction). For the U
 // component of benchmarks/cdu/src/cdu.f90:66-71,96-101 with the final
 // multiplication by one half (:39):
 //   x: Ax[(Ue+U0)^2 - (U0+Uw)^2] + 2Ax(Ue-Uw)U0 = Ax (Ue-Uw)(Ue+Uw+4U0)
-//   y: Ay[n vn - s vs] + (Ay/2)(n-s)(vn+vs)     = (Ay/2)[n(3vn+vs) - s(3vs+vn)]
+//   y: Ay[n vn - s vs] + (Ay/2)(n-s)(vn+vs)
+//        = (Ay/2)[2(n-s)(vn+vs) + (n+s)(vn-vs)]
 // where n, s are U's north and south face sums (U(j+1)+U, U+U(j-1)) and vn, vs
 // the V face sums at the same corners (V(i+1)+V at rows j and j-1); z is the y
 // form with U's top/bottom face sums and W's. The advective coefficients of the
 // reference (0.5/d along the component, 0.125/d across) are exactly 2A and A/2,
-// and Un-Us = n-s, so the flux and advective forms share every face sum. V and
-// W rotate the roles (compiler/tests/fixtures/stencils/{cvd,cdw}.f90:61-66,
-// 89-94). The tendency is -(1/2) of the sum, so each direction is one product
-// scaled by -A/2 (along the component) or -A/4 (across), accumulated by FMA.
+// and Un-Us = n-s, so the flux and advective forms share every sum. V and W
+// rotate the roles (compiler/tests/fixtures/stencils/{cvd,cdw}.f90:61-66,
+// 89-94). With every velocity in units of its direction's coefficient over x's,
+// the three directions of a component, and a scalar's six faces
+// (advection_point.cuh), are one sum of products times one coefficient.
 //
-// Scalars (this project's centred flux form, advection_point.cuh) regroup as
-//   -sum_d [c0 (Se+S0) - cw (S0+Sw)] = S0*D - sum_d (c0 Se - cw Sw),
-//   c = 0.5/d times the velocity at the face, D = sum_d (cw - c0),
-// with D shared by all scalars: 7 FP64 instructions per scalar instead of 11.
+// Precision: a field's values at a point's stencil keep 60 bits below the
+// largest of them (an FP64 operation 53 below its own operands), so that a
+// result is off by its two final roundings and 2^-56 or so of (largest
+// component value) x (largest velocity) in the stencil, whatever the tile.
+// Against extended precision the errors (2-norm and maximum) are 0.5 of the FP64
+// form's over the fields of the workloads, equal at worst. What the integers
+// cannot take (infinities, NaN, a value beside the point's own factors that is
+// far larger than they are) goes to FP64 point by point.
 //
-// Each point's own face sums (six, U(j+1)+U etc.) and scaled velocities (three)
-// are computed once and handed to the neighbours that need them: the x
-// neighbour by a warp shuffle, the y neighbour through a shared-memory row
-// exchange (an extra "edge" warp supplies the tile's south row and west
-// column), the level above in registers carried up the z-march. Results differ
-// from the reference's rounding by a few units in the last place of the
-// intermediate sums (measured max relative error ~1e-15 of each field's
-// maximum); the strict kernel stays the bit-exact default.
+// Each value is unpacked once, by the thread that owns its cell (the frame's by
+// the threads in turn), and read by its neighbours from shared memory. Values
+// two levels up are already on their way by asynchronous copies: held in
+// registers across the barrier instead, the loads cost 18-24 % of the step.
+// 8 warps of 128 registers, two CTAs per SM; with three (80 registers, spills)
+// 512 x 512 x 128 with three scalars took 1.79 ms instead of 1.54, 4-row tiles
+// 2.1, 16-row tiles 2.1 (each with its frame's share of the unpacking).
+// 512 x 512 x 128 with three scalars: 1.54 ms (the FP64 form 3.95); without
+// scalars 0.88; 257 x 193 x 61 with two, advanced: 170 us (475); 64 instances
+// with one scalar in one batched launch: 3.47 ms (9.43).
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "advection_faces.cuh"
 #include "advection_kernels.cuh"
+#include "wide_int.cuh"
 
 namespace f2c {
 
 constexpr int kFastTX = 32;        // points per tile along x (one warp)
 constexpr int kFastKZ = 32;        // levels per z-chunk for large grids
-constexpr int kFastSlots = 5;      // values exchanged per face row or column
+constexpr int kFastPrologue = 3;   // cost of a chunk's start, in half levels
 
-// Shared exchange of one level, double-buffered: the north-face values of
-// every row of the tile ([slot][row][lane], row 0 = the row south of the tile)
-// and the east-face values of the column west of the tile ([slot][row]).
-template <int TY>
+// Shared memory of a tile: the wide values (wide_int.cuh) of the tile's cells
+// and a one-cell frame, one plane per field and level in a ring of three levels
+// (the one below, of which a thread reads only its own cell; the level; the one
+// above it, being written), significands and exponents apart; and the FP64
+// values on their way from global memory, two levels of them, each read only by
+// the thread that asked for it.
+template <int NS, int TY>
 struct FastSmem {
-    static constexpr int SOUTH = kFastSlots * (TY + 1) * kFastTX;
-    static constexpr int WEST = kFastSlots * TY;
-    static constexpr int PER_BUFFER = SOUTH + WEST;
-    static constexpr int doubles = 2 * PER_BUFFER;
+    static constexpr int PITCH = kFastTX + 2, PLANE = (TY + 2) * PITCH;
+    static constexpr int FIELDS = 3 + NS;
+    static constexpr int FRAME = 2 * kFastTX + 2 * TY + 2;  // cells of the frame the stencils reach
+    static constexpr int THREADS = kFastTX * TY;
+    static constexpr int TURNS = (FIELDS * FRAME + THREADS - 1) / THREADS;
+    static constexpr int LEVEL = FIELDS * PLANE;
+    static constexpr int AHEAD = (FIELDS + TURNS) * THREADS;  // values on their way, a level
+    static constexpr int bytes = 8 * (3 * LEVEL + 2 * AHEAD) + 2 * 3 * LEVEL;
 };
 
 template <int TY>
-constexpr int fast_threads() { return kFastTX * (TY + 1); }
+constexpr int fast_threads() { return kFastTX * TY; }
 
-// CTAs per SM a tile height is compiled for by default: the register budget
-// follows (96 registers a thread at four 5-warp or two 9-warp CTAs, more at
-// one 17-warp CTA).
+// CTAs per SM a tile height is compiled for: 16 warps of 128 registers.
 template <int TY>
 constexpr int fast_ctas_per_sm() { return TY <= 4 ? 4 : (TY <= 8 ? 2 : 1); }
 
-// Tile height of the single-instance launches, and the CTAs per SM their
-// kernel is compiled for when the launch has at least kFastDeepCtas CTAs per
-// SM of work (72 registers; the three-scalar step then spills about 240 bytes
-// a thread, served by L1). More warps hide more of the FP64 and integer
-// latencies of large grids; measured at 512 x 512 x 128 with three
-// scalars, 8-row tiles took 4.10 ms at two CTAs per SM, 3.94 at three and 3.95
-// at four (4-row tiles 4.06, 4.03 and 4.03 at four, six and eight; 16-row
-// tiles 4.31 at one and 4.09 at two). Smaller launches keep two CTAs: at three
-// the 64 uneven instances of the ensemble, launched one at a time, ran 6 %
-// slower, and so did the serving ticks' batched steps.
-constexpr int kFastTY = 8;
-constexpr int kFastDeepCtasPerSM = 3;
-constexpr int kFastDeepCtas = 8;
+// Exponents above a field's own factors' at which it still keeps more bits than FP64: 60 - 5 of them.
+constexpr int kWideSlack = 5;
 
-// p(3q + qn) - pn(3qn + q): one direction of a momentum component across its
-// own axis, with p, pn the component's own face sums at the near and far face
-// and q, qn the other velocity's face sums at the same faces.
-__device__ __forceinline__ double cross_term(double p, double pn, double q, double qn) {
-    const double a = __fma_rn(3.0, q, qn);
-    const double b = __fma_rn(3.0, qn, q);
-    return __fma_rn(p, a, -pmul(pn, b));
+constexpr int kFastTY = 8;  // tile height of the single-instance launches
+
+// One momentum component in FP64 straight from memory. P is the component, d1
+// the stride along it; Q and R are the two other velocities, d2 and d3 the
+// strides along those. With n, s the component's face sums across an axis and
+// vn, vs the crossing velocity's, a direction is n(3vn+vs) - s(3vs+vn); along
+// the component (f1-f0)(f1+f0+4c).
+static __device__ double fast_component_fp64(const double *P, const double *Q, const double *R, long long d1,
+                                             long long d2, long long d3, double g, double c2, double c3,
+                                             double start) {
+    const double c = P[0];
+    auto cross = [&](const double *F, long long d) {
+        const double p = P[d] + c, pn = c + P[-d], q = F[d1] + F[0], qn = F[d1 - d] + F[-d];
+        return __fma_rn(p, __fma_rn(3.0, q, qn), -(pn * __fma_rn(3.0, qn, q)));
+    };
+    const double f1 = P[d1], f0 = P[-d1];
+    double t = __fma_rn(c3, cross(R, d3), start);
+    t = __fma_rn(c2, cross(Q, d2), t);
+    return __fma_rn(g, (f1 - f0) * __fma_rn(4.0, c, f1 + f0), t);
 }
 
-// (f1 - f0)(f1 + f0 + 4 c): the direction along a momentum component, from its
-// values one point either side (f1, f0) and at the point (c).
-__device__ __forceinline__ double along_term(double f1, double f0, double c) {
-    return pmul(f1 - f0, __fma_rn(4.0, c, f1 + f0));
+// The fields of `which` (bit n: U, V, W, scalars) at one point in FP64, for the
+// points whose stencil the wide integers cannot take (infinities, NaN,
+// subnormals, results near the ends of the exponent range) and for grids whose
+// coefficients they cannot. One call for a point: a call in each field's way
+// cost 10 % of the step.
+template <bool FILL, bool ADVANCE>
+static __device__ __noinline__ void fast_point_fp64(const AdvArgs &a, int i, int j, int k, unsigned which) {
+    const long long sx = a.sx, plane = a.plane;
+    const long long p = (long long)(i + a.h) + sx * (long long)(j + a.h) + plane * (long long)(k + a.h);
+    const double *U = a.u + p, *V = a.v + p, *W = a.w + p;
+    const FastCoefficients &c = a.f;
+    for (int f = 0; f < 3 + a.nscalar; ++f) {
+        double *out = f < 3 ? a.out[f] : a.st[f - 3];
+        if (!(which >> f & 1) || !out) continue;
+        const double *S = (f == 0 ? a.u : (f == 1 ? a.v : (f == 2 ? a.w : a.s[f - 3]))) + p;
+        const double start = ADVANCE ? S[0] : 0.0;
+        double t;
+        if (f == 0) {
+            t = fast_component_fp64(U, V, W, 1, sx, plane, c.gx, c.cy, c.cz, start);
+        } else if (f == 1) {
+            t = fast_component_fp64(V, U, W, sx, 1, plane, c.gy, c.cx, c.cz, start);
+        } else if (f == 2) {
+            t = fast_component_fp64(W, U, V, plane, 1, sx, c.gz, c.cx, c.cy, start);
+        } else {
+            const double e = c.sx * U[0], w = c.sx * U[-1], n = c.sy * V[0], s = c.sy * V[-sx], u = c.sz * W[0],
+                         b = c.sz * W[-plane];
+            t = __fma_rn(S[0], ((w - e) + (s - n)) + (b - u), start);
+            t = __fma_rn(-e, S[1], t);
+            t = __fma_rn(w, S[-1], t);
+            t = __fma_rn(-n, S[sx], t);
+            t = __fma_rn(s, S[-sx], t);
+            t = __fma_rn(-u, S[plane], t);
+            t = __fma_rn(b, S[-plane], t);
+        }
+        if (FILL) store_filled(out, f == 2 ? 1 : 0, a, i, j, k, t);
+        else out[p] = t;
+    }
 }
+
+// An 8-byte copy from global to shared memory that runs on while the thread does (cp.async).
+__device__ __forceinline__ void fetch(long long *to, const double *from) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from));
+}
+__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // One tile: columns [tile_x*32, +32) x [tile_y*TY, +TY) of the interior, levels
 // [k0, k1), for one output mode (ADVANCE: forward Euler, else the tendency).
-// Called by every thread of a (32, TY+1) block; `smem` holds
-// FastSmem<TY>::doubles. Starts and ends with the exchange buffers free.
+// Called by every thread of a (32, TY) block; `smem` holds
+// FastSmem<NS, TY>::bytes. Starts with the buffers free; a caller that goes on to
+// another tile has a barrier in between.
 template <int NS, int MASK, int TY, bool ADVANCE>
 __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int tile_y, int k0, int k1,
-                                               double *smem) {
-    constexpr bool DU = MASK & 1, DV = (MASK >> 1) & 1, DW = (MASK >> 2) & 1, DS = NS > 0;
+                                               long long *smem) {
+    constexpr bool DU = MASK & 1, DV = (MASK >> 1) & 1, DW = (MASK >> 2) & 1;
     constexpr bool filled = (MASK & kFillMask) != 0;  // F2C_ADVANCE_FILLED: outputs with their ghost images
-    // face sums each point computes (at its north/east/top faces)
-    constexpr bool F_UY = DU || DV, F_VX = DU || DV, F_UZ = DU || DW, F_WX = DU || DW, F_VZ = DV || DW,
-                   F_WY = DV || DW;
-    using Sm = FastSmem<TY>;
+    using Sm = FastSmem<NS, TY>;
+    constexpr int PITCH = Sm::PITCH, PLANE = Sm::PLANE, LEVEL = Sm::LEVEL, FIELDS = Sm::FIELDS;
     const int lane = threadIdx.x;
     const int warp = threadIdx.y;
-    const bool edge = warp == TY;
     const int i0 = tile_x * kFastTX, j0 = tile_y * TY;
     const int i = i0 + lane, j = j0 + warp;
-    const bool active = !edge && i < a.nx && j < a.ny;
-    const bool south_lane = edge && i < a.nx;                      // (i, j0-1)
-    const bool west_lane = edge && lane < TY && j0 + lane < a.ny;  // (i0-1, j0+lane)
+    const bool active = i < a.nx && j < a.ny;
+    const bool inside = i <= a.nx && j <= a.ny;  // cells the stencils reach
+    const bool across = i < a.h || i >= a.nx - a.h || j < a.h || j >= a.ny - a.h;
     const long long sx = a.sx, plane = a.plane;
-    const double *__restrict__ U = a.u;
-    const double *__restrict__ V = a.v;
-    const double *__restrict__ W = a.w;
-    const FastCoefficients c = a.f;
-    const int cj = edge ? j0 - 1 : j;
-    long long p = (long long)(i + a.h) + sx * (long long)(cj + a.h) + plane * (long long)(k0 + a.h);
-    long long pw = (long long)(i0 - 1 + a.h) + sx * (long long)(j0 + lane + a.h) + plane * (long long)(k0 + a.h);
-#define LD(A, q, di, dj, dk) __ldg((A) + (q) + (di) + (dj)*sx + (dk)*plane)
+    const FastCoefficients &c = a.f;
+    long long *const ring = smem;
+    long long *const ahead = smem + 3 * LEVEL + warp * kFastTX + lane;  // this thread's values on their way
+    short *const ring_e = reinterpret_cast<short *>(smem + 3 * LEVEL + 2 * Sm::AHEAD);
+    auto field = [&](int f) { return f == 0 ? a.u : (f == 1 ? a.v : (f == 2 ? a.w : a.s[f - 3])); };
+    auto put = [&](int at, int f, double x, auto scaled) {
+        Wide w = wide_pack(x, f < 3 ? c.wide_shift[f] : 0);
+        if (decltype(scaled)::value && (f == 1 || f == 2)) wide_scale(w, c.wide_ratio[f]);
+        ring[at] = w.m;
+        ring_e[at] = (short)w.e;
+    };
 
-    // values of the level below, carried up the march: face sums at the top faces of level k-1, W there,
-    // the vertical scaled velocity there, and this level's U, V, W (loaded as the level above).
-    double bUz = 0, bWx = 0, bVz = 0, bWy = 0, bcW = 0, Wm = 0, U0 = 0, V0 = 0, W0 = 0;
-    if (active) {
-        const double Um = LD(U, p, 0, 0, -1), Vm = LD(V, p, 0, 0, -1);
-        Wm = LD(W, p, 0, 0, -1);
-        U0 = LD(U, p, 0, 0, 0);
-        V0 = LD(V, p, 0, 0, 0);
-        W0 = LD(W, p, 0, 0, 0);
-        if (F_UZ) bUz = U0 + Um;
-        if (F_WX) bWx = LD(W, p, 1, 0, -1) + Wm;
-        if (F_VZ) bVz = V0 + Vm;
-        if (F_WY) bWy = LD(W, p, 0, 1, -1) + Wm;
-        if (DS) bcW = c.sz * Wm;
+    // The frame around the tile (the rows south and north of it, its west and east columns, the corners U
+    // north-west and V south-east): one value of one field to each of the first FIELDS * FRAME turns of the threads.
+    constexpr int TURNS = Sm::TURNS;
+    const double *frame_at[TURNS];
+    int frame_to[TURNS], frame_field[TURNS];
+#pragma unroll
+    for (int t = 0; t < TURNS; ++t) {
+        const int n = t * kFastTX * TY + warp * kFastTX + lane;
+        const int f = n / Sm::FRAME, m = n - f * Sm::FRAME;
+        const int r = m - 2 * kFastTX;
+        const int row = m < kFastTX ? -1 : (r < 0 ? TY : (r < TY ? r : (r < 2 * TY ? r - TY : (r == 2 * TY ? TY : -1))));
+        const int col = r < 0 ? (m & (kFastTX - 1)) : (r < TY || r == 2 * TY ? -1 : kFastTX);
+        const bool use = f < FIELDS && i0 + col <= a.nx && j0 + row <= a.ny;
+        const double *base = a.u;
+#pragma unroll
+        for (int g = 1; g < FIELDS; ++g)
+            if (f == g) base = field(g);
+        frame_at[t] = base + (i0 + col + a.h) + sx * (long long)(j0 + row + a.h) + plane * (long long)(k0 - 1 + a.h);
+        frame_to[t] = use ? f * PLANE + (row + 1) * PITCH + col + 1 : -1;
+        frame_field[t] = f;
     }
-
-    int buf = 0;
-    for (int k = k0; k < k1; ++k, p += plane, pw += plane, buf ^= 1) {
-        double *south = smem + buf * Sm::PER_BUFFER;  // [slot][TY+1][32]
-        double *west = south + Sm::SOUTH;             // [slot][TY]
-        constexpr int ROW = kFastTX, SLOT = (TY + 1) * kFastTX;
-        // ---------------- own faces, handed to the neighbours ----------------
-        double Up = 0, Vp = 0, Wp = 0;
-        double sUy = 0, sVx = 0, sUz = 0, sWx = 0, sVz = 0, sWy = 0, cU = 0, cV = 0, cW = 0;
-        if (active) {
-            Up = LD(U, p, 0, 0, 1);
-            Vp = LD(V, p, 0, 0, 1);
-            Wp = LD(W, p, 0, 0, 1);
-            if (F_UY) sUy = LD(U, p, 0, 1, 0) + U0;
-            if (F_VX) sVx = LD(V, p, 1, 0, 0) + V0;
-            if (F_UZ) sUz = Up + U0;
-            if (F_WX) sWx = LD(W, p, 1, 0, 0) + W0;
-            if (F_VZ) sVz = Vp + V0;
-            if (F_WY) sWy = LD(W, p, 0, 1, 0) + W0;
-            if (DS) {
-                cU = pmul(c.sx, U0);
-                cV = pmul(c.sy, V0);
-                cW = pmul(c.sz, W0);
-            }
-            const int at = (warp + 1) * ROW + lane;
-            if (DU) {
-                south[0 * SLOT + at] = sUy;
-                south[1 * SLOT + at] = sVx;
-            }
-            if (DW) {
-                south[2 * SLOT + at] = sWy;
-                south[3 * SLOT + at] = sVz;
-            }
-            if (DS) south[4 * SLOT + at] = cV;
-        } else if (edge) {
-            if (south_lane) {
-                // north faces of row j0-1: the tile's south faces
-                if (DU || DW) {
-                    const double u0 = LD(U, p, 0, 0, 0), v0 = LD(V, p, 0, 0, 0);
-                    if (DU) {
-                        south[0 * SLOT + lane] = LD(U, p, 0, 1, 0) + u0;
-                        south[1 * SLOT + lane] = LD(V, p, 1, 0, 0) + v0;
-                    }
-                    if (DW) {
-                        south[2 * SLOT + lane] = LD(W, p, 0, 1, 0) + LD(W, p, 0, 0, 0);
-                        south[3 * SLOT + lane] = LD(V, p, 0, 0, 1) + v0;
-                    }
-                    if (DS) south[4 * SLOT + lane] = c.sy * v0;
-                } else if (DS) {
-                    south[4 * SLOT + lane] = c.sy * LD(V, p, 0, 0, 0);
-                }
-            }
-            if (west_lane) {
-                // east faces of column i0-1 (row j0+lane): the tile's west faces
-                if (DV || DW) {
-                    const double u0 = LD(U, pw, 0, 0, 0);
-                    if (DV) {
-                        west[0 * TY + lane] = LD(V, pw, 1, 0, 0) + LD(V, pw, 0, 0, 0);
-                        west[1 * TY + lane] = LD(U, pw, 0, 1, 0) + u0;
-                    }
-                    if (DW) {
-                        west[2 * TY + lane] = LD(W, pw, 1, 0, 0) + LD(W, pw, 0, 0, 0);
-                        west[3 * TY + lane] = LD(U, pw, 0, 0, 1) + u0;
-                    }
-                    if (DS) west[4 * TY + lane] = c.sx * u0;
-                } else if (DS) {
-                    west[4 * TY + lane] = c.sx * LD(U, pw, 0, 0, 0);
-                }
+    const int own = (warp + 1) * PITCH + lane + 1;
+    const long long p0 = (long long)(i + a.h) + sx * (long long)(j + a.h) + plane * (long long)(k0 + a.h);
+    long long p = p0;
+    // the values of level k (offset `at` from level k0's), into half `half` of the buffer
+    auto fetch_level = [&](long long *to, long long at, long long frame_step) {
+        if (inside) {
+#pragma unroll
+            for (int f = 0; f < FIELDS; ++f) fetch(to + f * Sm::THREADS, field(f) + at);
+        }
+#pragma unroll
+        for (int t = 0; t < TURNS; ++t) {
+            if (frame_to[t] >= 0) {
+                fetch(to + (FIELDS + t) * Sm::THREADS, frame_at[t]);
+                frame_at[t] += frame_step;
             }
         }
-        // x neighbours by shuffle (every lane of a compute warp takes part; lane 0 reads the west column below)
-        double wVx = 0, wUy = 0, wWx = 0, wUz = 0, wcU = 0;
-        if (!edge) {
-            if (DV) {
-                wVx = __shfl_up_sync(0xffffffffu, sVx, 1);
-                wUy = __shfl_up_sync(0xffffffffu, sUy, 1);
-            }
-            if (DW) {
-                wWx = __shfl_up_sync(0xffffffffu, sWx, 1);
-                wUz = __shfl_up_sync(0xffffffffu, sUz, 1);
-            }
-            if (DS) wcU = __shfl_up_sync(0xffffffffu, cU, 1);
+        fetch_commit();
+    };
+    auto put_level_as = [&](const long long *from, int to, auto scaled) {
+        if (inside) {
+#pragma unroll
+            for (int f = 0; f < FIELDS; ++f) put(to + f * PLANE + own, f, __longlong_as_double(from[f * Sm::THREADS]), scaled);
+        }
+#pragma unroll
+        for (int t = 0; t < TURNS; ++t) {
+            if (frame_to[t] >= 0)
+                put(to + frame_to[t], frame_field[t], __longlong_as_double(from[(FIELDS + t) * Sm::THREADS]), scaled);
+        }
+    };
+    auto put_level = [&](const long long *from, int to) {
+        if (c.wide_scaled) put_level_as(from, to, std::true_type{});
+        else put_level_as(from, to, std::false_type{});
+    };
+    // levels k0-1 (slot 2: own column, and W's frame) and k0 (slot 0); level k0+1 on its way
+    Wide wem{0, 0}, wnm{0, 0};
+    fetch_level(ahead, p - plane, plane);
+    fetch_level(ahead + Sm::AHEAD, p, plane);
+    fetch_wait<1>();
+    put_level(ahead, 2 * LEVEL);
+    fetch_level(ahead, p + plane, plane);
+    fetch_wait<1>();
+    put_level(ahead + Sm::AHEAD, 0);
+    if (DU || DV) {
+        __syncthreads();
+        const int n = 2 * LEVEL + 2 * PLANE + own;
+        wem = {ring[n + 1], ring_e[n + 1]};
+        wnm = {ring[n + PITCH], ring_e[n + PITCH]};
+    }
+
+    int below = 2, slot = 0;  // ring slots of levels k-1 and k
+    int half = 0;             // of the buffer, with level k+1
+    for (int k = k0; k < k1; ++k, p += plane, half ^= 1) {
+        const int above = 3 - below - slot;
+        // level k+2 on its way, and level k+1 into the ring
+        if (k + 1 < k1) fetch_level(ahead + (half ^ 1) * Sm::AHEAD, p + 2 * plane, plane);
+        else fetch_commit();
+        fetch_wait<1>();
+        put_level(ahead + half * Sm::AHEAD, above * LEVEL);
+        double old[ADVANCE ? FIELDS : 1];  // the fields' values, asked for ahead of their use
+        if (ADVANCE && active) {
+#pragma unroll
+            for (int f = 0; f < FIELDS; ++f) old[f] = ldg_again(field(f) + p);
         }
         __syncthreads();
-        // ---------------- the tendencies ----------------
         if (active) {
-            if (lane == 0) {
-                if (DV) {
-                    wVx = west[0 * TY + warp];
-                    wUy = west[1 * TY + warp];
-                }
-                if (DW) {
-                    wWx = west[2 * TY + warp];
-                    wUz = west[3 * TY + warp];
-                }
-                if (DS) wcU = west[4 * TY + warp];
-            }
-            const int at = warp * ROW + lane;  // the row south of this one
+            const long long *now = ring + slot * LEVEL + own, *next = ring + above * LEVEL + own,
+                            *prev = ring + below * LEVEL + own;
+            const short *now_e = ring_e + slot * LEVEL + own, *next_e = ring_e + above * LEVEL + own,
+                      *prev_e = ring_e + below * LEVEL + own;
+            auto at = [&](int f, int row, int col) {
+                const int n = f * PLANE + row * PITCH + col;
+                return Wide{now[n], now_e[n]};
+            };
+            auto over = [&](int f, int row, int col) {
+                const int n = f * PLANE + row * PITCH + col;
+                return Wide{next[n], next_e[n]};
+            };
+            auto under = [&](int f) { return Wide{prev[f * PLANE], prev_e[f * PLANE]}; };
+            const Wide z{0, 0};
+            // the stencil of U, V and W, each field aligned to its own largest exponent in it
+            const Wide u0 = at(0, 0, 0), v0 = at(1, 0, 0), w0 = at(2, 0, 0);
+            const Wide uw = at(0, 0, -1), un = DU || DV ? at(0, 1, 0) : z, up = DU || DW ? over(0, 0, 0) : z;
+            const Wide ue = DU ? at(0, 0, 1) : z, us = DU ? at(0, -1, 0) : z, um = DU ? under(0) : z;
+            const Wide uwn = DV ? at(0, 1, -1) : z, uwp = DW ? over(0, 0, -1) : z;
+            const Wide vs = at(1, -1, 0), ve = DU || DV ? at(1, 0, 1) : z, vp = DV || DW ? over(1, 0, 0) : z;
+            const Wide vn = DV ? at(1, 1, 0) : z, vw = DV ? at(1, 0, -1) : z, vm = DV ? under(1) : z;
+            const Wide ves = DU ? at(1, -1, 1) : z, vsp = DW ? over(1, -1, 0) : z;
+            const Wide wm = under(2), we = DU || DV || DW ? at(2, 0, 1) : z, wn = DU || DV || DW ? at(2, 1, 0) : z;
+            const Wide ww = DW ? at(2, 0, -1) : z, ws = DW ? at(2, -1, 0) : z, wp = DW ? over(2, 0, 0) : z;
+            // (pu, pv, pw: over the component's own part of it)
+            const int pu = max3(max3(u0.e, uw.e, up.e), max3(un.e, ue.e, us.e), um.e), EU = max3(pu, uwn.e, uwp.e);
+            const int pv = max3(max3(v0.e, vs.e, vp.e), max3(vn.e, ve.e, vw.e), vm.e), EV = max3(pv, ves.e, vsp.e);
+            const int pw = max3(max3(w0.e, wm.e, wp.e), max3(wn.e, we.e, ww.e), ws.e), EW = max3(pw, wem.e, wnm.e);
+            const int E = max3(EU, EV, EW);
+            const int du = E - EU, dv = E - EV, dw = E - EW;
+            const int tu = EU + 3, tv = EV + 3, tw = EW + 3;
+            const long long au0 = wide_align(u0, tu), auw = wide_align(uw, tu), aun = wide_align(un, tu),
+                            aup = wide_align(up, tu);
+            const long long av0 = wide_align(v0, tv), avs = wide_align(vs, tv), ave = wide_align(ve, tv),
+                            avp = wide_align(vp, tv);
+            const long long aw0 = wide_align(w0, tw), awm = wide_align(wm, tw), awe = wide_align(we, tw),
+                            awn = wide_align(wn, tw);
+            // a component's or scalar's value from its sum T at exponent e, stored; `slow` notes what does not fit,
+            // and what is computed at a scale above 2^kWideSlack times its own largest factors' (`used`): next to a
+            // value much larger than the ones that it reads itself
+            unsigned slow = 0;
+            // whether the new value has ghost images (store_filled), or is a W wall face
+            const bool images = filled && (across || k < a.h || k >= a.nz - 1 - a.h);
+            auto finish = [&](int f, long long T, int e, int used) {
+                const int g = f < 3 ? f : 3;
+                double *o = f < 3 ? a.out[f] : a.st[f - 3];
+                bool fits;
+                double t = wide_result(T, e, c.wide_hi[g], c.wide_lo[g], c.wide_e[g], fits);
+                if (!fits || e - used > kWideSlack) slow |= 1u << f;
+                if (ADVANCE) t += old[ADVANCE ? f : 0];
+                if (!o) return;
+                if (images) store_filled(o, f == 2 ? 1 : 0, a, i, j, k, t);
+                else o[p] = t;
+            };
             if (DU) {
-                const double X = along_term(LD(U, p, 1, 0, 0), LD(U, p, -1, 0, 0), U0);
-                const double Y = cross_term(sUy, south[0 * SLOT + at], sVx, south[1 * SLOT + at]);
-                const double Z = cross_term(sUz, bUz, sWx, bWx);
-                double t = ADVANCE ? __fma_rn(c.cz, Z, U0) : pmul(c.cz, Z);
-                t = __fma_rn(c.cy, Y, t);
-                t = __fma_rn(c.gx, X, t);
-                if (a.out[0]) { if (filled) store_filled(a.out[0], 0, a, i, j, k, t); else a.out[0][p] = t; }
+                const long long aue = wide_align(ue, tu), aus = wide_align(us, tu), aum = wide_align(um, tu);
+                const long long q = av0 + ave, qs = avs + wide_align(ves, tv);
+                const long long r = aw0 + awe, rb = awm + wide_align(wem, tw);
+                const long long T = wide_component(aue, auw, aun, aus, aup, aum, au0, du, q, qs, dv, r, rb, dw);
+                finish(0, T, EU + E, pu + max3(max3(ue.e, uw.e, v0.e), max3(ve.e, vs.e, ves.e), max(max3(w0.e, we.e, wm.e), wem.e)));
             }
             if (DV) {
-                const double X = cross_term(sVx, wVx, sUy, wUy);
-                const double Y = along_term(LD(V, p, 0, 1, 0), LD(V, p, 0, -1, 0), V0);
-                const double Z = cross_term(sVz, bVz, sWy, bWy);
-                double t = ADVANCE ? __fma_rn(c.cz, Z, V0) : pmul(c.cz, Z);
-                t = __fma_rn(c.gy, Y, t);
-                t = __fma_rn(c.cx, X, t);
-                if (a.out[1]) { if (filled) store_filled(a.out[1], 0, a, i, j, k, t); else a.out[1][p] = t; }
+                const long long avn = wide_align(vn, tv), avw = wide_align(vw, tv), avm = wide_align(vm, tv);
+                const long long q = au0 + aun, qw = auw + wide_align(uwn, tu);
+                const long long r = aw0 + awn, rb = awm + wide_align(wnm, tw);
+                const long long T = wide_component(avn, avs, ave, avw, avp, avm, av0, dv, q, qw, du, r, rb, dw);
+                finish(1, T, EV + E, pv + max3(max3(vn.e, vs.e, u0.e), max3(un.e, uw.e, uwn.e), max(max3(w0.e, wn.e, wm.e), wnm.e)));
             }
             if (DW) {
-                const double X = cross_term(sWx, wWx, sUz, wUz);
-                const double Y = cross_term(sWy, south[2 * SLOT + at], sVz, south[3 * SLOT + at]);
-                const double Z = along_term(Wp, Wm, W0);
-                double t = ADVANCE ? __fma_rn(c.gz, Z, W0) : pmul(c.gz, Z);
-                t = __fma_rn(c.cy, Y, t);
-                t = __fma_rn(c.cx, X, t);
-                if (a.out[2]) { if (filled) store_filled(a.out[2], 1, a, i, j, k, t); else a.out[2][p] = t; }
+                const long long awp = wide_align(wp, tw), aww = wide_align(ww, tw), aws = wide_align(ws, tw);
+                const long long q = au0 + aup, qw = auw + wide_align(uwp, tu);
+                const long long r = av0 + avp, rs = avs + wide_align(vsp, tv);
+                const long long T = wide_component(awp, awm, awe, aww, awn, aws, aw0, dw, q, qw, du, r, rs, dv);
+                finish(2, T, EW + E, pw + max3(max3(wp.e, wm.e, u0.e), max3(up.e, uw.e, uwp.e), max(max3(v0.e, vp.e, vs.e), vsp.e)));
             }
-            if (DS) {
-                const double scV = south[4 * SLOT + at];
-                const double D = ((wcU - cU) + (scV - cV)) + (bcW - cW);
+            wem = we;
+            wnm = wn;
+            if (NS > 0) {
+                const int faces = max(max3(u0.e, uw.e, v0.e), max3(vs.e, w0.e, wm.e));
+                const long long east = wide_shift(au0, du), west = -wide_shift(auw, du), north = wide_shift(av0, dv),
+                                south = -wide_shift(avs, dv), top = wide_shift(aw0, dw), bottom = -wide_shift(awm, dw);
 #pragma unroll
                 for (int n = 0; n < NS; ++n) {
-                    const double *__restrict__ S = a.s[n];
-                    const double S0 = LD(S, p, 0, 0, 0);
-                    double t = ADVANCE ? __fma_rn(S0, D, S0) : pmul(S0, D);
-                    t = __fma_rn(-cU, LD(S, p, 1, 0, 0), t);
-                    t = __fma_rn(wcU, LD(S, p, -1, 0, 0), t);
-                    t = __fma_rn(-cV, LD(S, p, 0, 1, 0), t);
-                    t = __fma_rn(scV, LD(S, p, 0, -1, 0), t);
-                    t = __fma_rn(-cW, LD(S, p, 0, 0, 1), t);
-                    t = __fma_rn(bcW, LD(S, p, 0, 0, -1), t);
-                    if (a.st[n]) { if (filled) store_filled(a.st[n], 0, a, i, j, k, t); else a.st[n][p] = t; }
+                    const Wide s0 = at(3 + n, 0, 0), se = at(3 + n, 0, 1), sw = at(3 + n, 0, -1), sn = at(3 + n, 1, 0),
+                               ss = at(3 + n, -1, 0), sp = over(3 + n, 0, 0), sm = under(3 + n);
+                    const int ES = max3(max3(s0.e, se.e, sw.e), max3(sn.e, ss.e, sp.e), sm.e), ts = ES + 2;
+                    const long long as0 = wide_align(s0, ts);
+                    WideSum sum;
+                    sum.add(east, wide_align(se, ts) + as0);
+                    sum.add(west, wide_align(sw, ts) + as0);
+                    sum.add(north, wide_align(sn, ts) + as0);
+                    sum.add(south, wide_align(ss, ts) + as0);
+                    sum.add(top, wide_align(sp, ts) + as0);
+                    sum.add(bottom, wide_align(sm, ts) + as0);
+                    finish(3 + n, sum.value(), ES + E, ES + faces);
                 }
             }
-            // carry up the march
-            bUz = sUz; bWx = sWx; bVz = sVz; bWy = sWy; bcW = cW;
-            Wm = W0;
-            U0 = Up; V0 = Vp; W0 = Wp;
+            if (E >= c.wide_limit) slow = ~0u;
+            if (slow) fast_point_fp64<filled, ADVANCE>(a, i, j, k, slow);
         }
+        below = slot;
+        slot = above;
     }
-#undef LD
 }
 
 // The tile in the instance's output mode. The mode is a template argument of
@@ -305,7 +385,8 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
 // (pmul, off the FP64 pipe) rather than an FMA with a zero addend, which a
 // runtime choice would leave on the FP64 pipe; a filled advance is an advance.
 template <int NS, int MASK, int TY>
-__device__ __forceinline__ void fast_tile(const AdvArgs &a, int tile_x, int tile_y, int k0, int k1, double *smem) {
+__device__ __forceinline__ void fast_tile(const AdvArgs &a, int tile_x, int tile_y, int k0, int k1,
+                                          long long *smem) {
     if constexpr ((MASK & kFillMask) != 0) {
         fast_tile_mode<NS, MASK, TY, true>(a, tile_x, tile_y, k0, k1, smem);
     } else if (a.mode != 0) {
@@ -316,34 +397,46 @@ __device__ __forceinline__ void fast_tile(const AdvArgs &a, int tile_x, int tile
 }
 
 template <int NS, int MASK, int TY, int CTAS = fast_ctas_per_sm<TY>()>
-__global__ void __launch_bounds__(fast_threads<TY>(), CTAS) advection_fast_kernel(const AdvArgs a) {
-    __shared__ double smem[FastSmem<TY>::doubles];
+__global__ void __launch_bounds__(fast_threads<TY>(), CTAS)
+    advection_fast_kernel(const __grid_constant__ AdvArgs a) {
+    extern __shared__ long long wide_smem[];
     const int k0 = blockIdx.z * a.kz;
-    fast_tile<NS, MASK, TY>(a, blockIdx.x, blockIdx.y, k0, min(k0 + a.kz, a.nz), smem);
+    fast_tile<NS, MASK, TY>(a, blockIdx.x, blockIdx.y, k0, min(k0 + a.kz, a.nz), wide_smem);
 }
 
-// z-chunk depth of one launch: deep for large grids, shallower for small ones
-// so that at least four CTAs per SM are available (down to two levels).
+// z-chunk depth of one launch: the one that takes the fewest level-times, waves
+// of CTAs times the levels of a chunk and its start (two levels unpacked before
+// the first is computed, about a level and a half of time); of equal ones the
+// deepest. 256 x 256 x 64: 14 levels, 121 us (8 levels, as four CTAs per SM would
+// have, 131); 150 x 100 x 50: 7 levels, 29 us (4: 31, 8: 33).
 inline int fast_chunk_depth(int nx, int ny, int nz, int ty, int sms) {
     const long long tiles = (long long)((nx + kFastTX - 1) / kFastTX) * ((ny + ty - 1) / ty);
-    const long long want = 4LL * (sms > 0 ? sms : 152);
-    long long kz = (tiles * nz + want - 1) / want;
-    if (kz > kFastKZ) kz = kFastKZ;
-    if (kz < 2) kz = 2;
-    return (int)kz;
+    const long long slots = (long long)(sms > 0 ? sms : 152) * fast_ctas_per_sm<kFastTY>();
+    long long best = -1;
+    int depth = 1;
+    for (int kz = 1; kz <= kFastKZ && kz <= nz; ++kz) {
+        const long long waves = (tiles * ((nz + kz - 1) / kz) + slots - 1) / slots;
+        const long long cost = waves * (2 * kz + kFastPrologue);
+        if (best < 0 || cost <= best) {
+            best = cost;
+            depth = kz;
+        }
+    }
+    return depth;
 }
 
 template <int NS, int MASK, int TY>
 cudaError_t launch_fast(const AdvArgs &a, int sms, cudaStream_t stream) {
+    using Sm = FastSmem<NS, TY>;
     AdvArgs b = a;
     if (b.kz <= 0) b.kz = fast_chunk_depth(b.nx, b.ny, b.nz, TY, sms);
-    const dim3 block(kFastTX, TY + 1, 1);
+    static std::atomic<unsigned long long> configured{0};
+    const auto kernel = advection_fast_kernel<NS, MASK, TY>;
+    const cudaError_t e = configure_shared_once(configured, (const void *)kernel, Sm::bytes);
+    if (e != cudaSuccess) return e;
+    const dim3 block(kFastTX, TY, 1);
     const dim3 grid((b.nx + kFastTX - 1) / kFastTX, (b.ny + TY - 1) / TY, (b.nz + b.kz - 1) / b.kz);
-    const long long ctas = (long long)grid.x * grid.y * grid.z;
-    if (TY == kFastTY && ctas >= (long long)kFastDeepCtas * (sms > 0 ? sms : 152))
-        advection_fast_kernel<NS, MASK, TY, kFastDeepCtasPerSM><<<grid, block, 0, stream>>>(b);
-    else
-        advection_fast_kernel<NS, MASK, TY><<<grid, block, 0, stream>>>(b);
+    kernel<<<grid, block, Sm::bytes, stream>>>(b);
     return cudaGetLastError();
 }
 

@@ -70,7 +70,7 @@ template <int NS, int MASK, int TY>
 __global__ void __launch_bounds__(fast_threads<TY>(), fast_ctas_per_sm<TY>())
     advection_batched_fast_kernel(const AdvArgs *__restrict__ instances, const BatchItem *__restrict__ items,
                                   int nitems, unsigned *counter) {
-    __shared__ double smem[FastSmem<TY>::doubles];
+    extern __shared__ long long wide_smem[];
     __shared__ int slot;
     __shared__ AdvArgs args;
     for (;;) {
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(fast_threads<TY>(), fast_ctas_per_sm<TY>())
         const BatchItem it = items[n];
         stage_args(&args, instances + it.instance);
         __syncthreads();
-        fast_tile<NS, MASK, TY>(args, it.tile_x, it.tile_y, it.k0, it.k1, smem);
+        fast_tile<NS, MASK, TY>(args, it.tile_x, it.tile_y, it.k0, it.k1, wide_smem);
     }
 }
 
@@ -92,13 +92,21 @@ struct Kernel {
     cudaError_t status;
 };
 
+template <int NS, int MASK, int TY>
+Kernel fast_kernel() {
+    using Sm = FastSmem<NS, TY>;
+    static std::atomic<unsigned long long> configured{0};
+    const void *fn = (const void *)advection_batched_fast_kernel<NS, MASK, TY>;
+    return {fn, Sm::bytes, configure_shared_once(configured, fn, Sm::bytes)};
+}
+
 template <int NS, int MASK>
 Kernel kernel_of(bool fast, int rows) {
     if (fast) {
         switch (rows) {
-        case 4: return {(const void *)advection_batched_fast_kernel<NS, MASK, 4>, 0, cudaSuccess};
-        case 16: return {(const void *)advection_batched_fast_kernel<NS, MASK, 16>, 0, cudaSuccess};
-        default: return {(const void *)advection_batched_fast_kernel<NS, MASK, 8>, 0, cudaSuccess};
+        case 4: return fast_kernel<NS, MASK, 4>();
+        case 16: return fast_kernel<NS, MASK, 16>();
+        default: return fast_kernel<NS, MASK, 8>();
         }
     }
     static std::atomic<unsigned long long> configured{0};
@@ -265,7 +273,7 @@ int finish(const Built &b, int32_t count, void *workspace, size_t workspace_byte
         const Kernel k = kernel_for(b.ns, b.mask, fast, b.rows);
         if (k.status != cudaSuccess) return fail(6, std::string("batch kernel set-up: ") + cudaGetErrorString(k.status));
         int n = 0;
-        const int threads = kFaceTX * (b.rows + 1);
+        const int threads = kFaceTX * (fast ? b.rows : b.rows + 1);
         const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k.fn, threads, k.smem);
         if (e != cudaSuccess || n < 1) return fail(6, "batch kernel does not fit on an SM");
         per_sm = std::min(per_sm, n);
@@ -406,7 +414,7 @@ extern "C" int f2c_batch_step_v1(const f2c_batch_plan_v1 *plan, void *stream) {
     if (k.status != cudaSuccess) return fail(6, std::string("batch kernel set-up: ") + cudaGetErrorString(k.status));
     int nitems = plan->items;
     void *args[] = {(void *)&descs, (void *)&items, (void *)&nitems, (void *)&counter};
-    e = cudaLaunchKernel(k.fn, dim3(plan->ctas), dim3(kFaceTX, rows + 1, 1), args, k.smem, s);
+    e = cudaLaunchKernel(k.fn, dim3(plan->ctas), dim3(kFaceTX, fast ? rows : rows + 1, 1), args, k.smem, s);
     if (e != cudaSuccess) return fail(6, std::string("batch launch: ") + cudaGetErrorString(e));
     return 0;
 }

@@ -1,0 +1,147 @@
+// Stencil arithmetic in 64-bit fixed point at the stencil's own scale.
+//
+// GB300 issues FP64 at 1.68 lane operations per clock per SM; a 64-bit addition
+// is one integer instruction and a 32 x 32 + 64 multiplication another, 64 lanes
+// each. A sum of products over neighbouring values therefore costs less in
+// integers, provided that they share a scale: FP64 values are unpacked to a
+// signed significand and an exponent (Wide), the values of one field that a
+// point reads are shifted to the largest exponent among them (wide_align), added
+// as integers, and multiplied to the leading 64 bits of the products' sum
+// (WideSum), which one conversion and one FP64 product bring back (wide_result).
+// No rounding depends on the order of the terms, or on which tile has the point.
+//
+// Ranges. An unpacked |m| is below 2^63, aligned with a headroom of h bits below
+// 2^(63-h). With h = 3: two values' sum or difference is below 2^61, the sums of
+// four below 2^62, f1 + f0 + 4c below 6 x 2^60; a product's high words stay
+// below 2^60.6 and its middle ones (the low word's upper 29 bits) below 2^60.4,
+// so that a component's five products add up below 2^62.7 in both. A scalar's
+// values have h = 2, its velocities 3: six products of 2^58, middle words of 2^59.
+// Dropped: the value bits beyond the alignment's 60 (61), three bits of each low
+// word and the low words' product, together at most 27 and about one unit of
+// 2^-56 times (power of two above the largest component value) times (that of
+// the largest velocity).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace f2c {
+
+constexpr int kWideSpecial = 8192;  // the exponent of infinities and NaN
+
+struct Wide {
+    long long m;  // signed significand: 53 bits from bit 62 down
+    int e;        // biased exponent (of the value times 2^n, see wide_pack)
+};
+
+// x * 2^n: a negative significand one's complemented (2^-62 of it off), zero and
+// subnormals without the leading bit, infinities and NaN as kWideSpecial.
+__device__ __forceinline__ Wide wide_pack(double x, int n) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int e = (int)((hi >> 20) & 0x7ffu);
+    const long long s = (long long)((int)hi >> 31);
+    Wide r;
+    r.e = e + n;
+    r.m = (long long)((((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo) << 10) ^ s;
+    if ((unsigned)(e - 1) >= 2046u) {
+        if (e == 0) {
+            r.e = 1 + n;
+            r.m = (long long)((((unsigned long long)(hi & 0xfffffu) << 32) | lo) << 10) ^ s;
+        } else {
+            r.e = kWideSpecial;
+        }
+    }
+    return r;
+}
+
+// m >> n for any n >= 0 (the PTX shift stops at the width).
+__device__ __forceinline__ long long wide_shift(long long m, int n) {
+    long long r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(m), "r"(n));
+    return r;
+}
+
+// The significand at the exponent top - headroom: top is the largest exponent of the stencil plus the headroom.
+__device__ __forceinline__ long long wide_align(Wide a, int top) { return wide_shift(a.m, top - a.e); }
+
+__device__ __forceinline__ int max3(int a, int b, int c) { return __vimax3_s32(a, b, c); }
+
+// The words of a significand as 32-bit integers: the high one, and the low one's
+// upper 29 bits. Inline PTX, so that the compiler sees plain 32-bit operands and
+// multiplies them by the one-instruction 32 x 32 + 64 form; from shifts it knows
+// the ranges of, it builds 64 x 64 products instead (16 instructions for 5).
+__device__ __forceinline__ int wide_high(long long m) {
+    int r;
+    asm("{.reg .b32 t; mov.b64 {t, %0}, %1;}" : "=r"(r) : "l"(m));
+    return r;
+}
+__device__ __forceinline__ int wide_low(long long m) {
+    int r;
+    asm("{.reg .b32 t, u; mov.b64 {t, u}, %1; shr.u32 %0, t, 3;}" : "=r"(r) : "l"(m));
+    return r;
+}
+
+// m + m as one 64-bit addition (the compiler's own choice, a shift, is two instructions).
+__device__ __forceinline__ long long wide_twice(long long m) {
+    long long r;
+    asm("add.s64 %0, %1, %1;" : "=l"(r) : "l"(m));
+    return r;
+}
+
+// A sum of products' leading 64 bits.
+struct WideSum {
+    long long high = 0, middle = 0;
+    __device__ __forceinline__ void add(long long a, long long b) {
+        const int ah = wide_high(a), bh = wide_high(b);
+        const int al = wide_low(a), bl = wide_low(b);
+        high += (long long)ah * bh;
+        middle += (long long)ah * bl;
+        middle += (long long)al * bh;
+    }
+    __device__ __forceinline__ long long value() const { return high + (middle >> 29); }
+};
+
+// A momentum component's sum: f1, f0 and c along it (one cell either side, and
+// the point), a1, a0 and b1, b0 across its two other axes, q, qn (r, rn) the
+// crossing velocity's face sums at the two faces of that axis, each shifted by
+// its field's distance from the largest exponent:
+//   2[(f1-f0)(f1+f0+4c) + (a1-a0)(q+qn) + (b1-b0)(r+rn)] + (a1+a0+2c)(q-qn) + (b1+b0+2c)(r-rn).
+__device__ __forceinline__ long long wide_component(long long f1, long long f0, long long a1, long long a0, long long b1,
+                                                    long long b0, long long c, int d, long long q, long long qn, int dq,
+                                                    long long r, long long rn, int dr) {
+    WideSum s;
+    const long long c2 = wide_twice(c);
+    s.add(wide_shift(f1 - f0, d), (f1 + f0) + wide_twice(c2));
+    s.add(a1 - a0, wide_shift(q + qn, dq));
+    s.add(b1 - b0, wide_shift(r + rn, dr));
+    s.high = wide_twice(s.high);
+    s.middle = wide_twice(s.middle);
+    s.add((a1 + a0) + c2, wide_shift(q - qn, dq));
+    s.add((b1 + b0) + c2, wide_shift(r - rn, dr));
+    return s.value();
+}
+
+// A packed value times a ratio in (1/2, 1) given as `r` = ratio * 2^62, a
+// multiple of 8 (so that the sum's dropped bits are zero): 2^-59 of it off.
+__device__ __forceinline__ void wide_scale(Wide &w, long long r) {
+    WideSum s;
+    s.add(w.m, r);
+    w.m = s.value() << 2;
+}
+
+// T * 2^e * k, for the coefficient k whose words are `khi`, `klo` with the sum's
+// constant 2^-offset taken off the exponent field; `ke` is that field less one.
+// The conversion rounds T to 53 bits, the product rounds once more. Where the
+// factor is below the normal range the product is taken 2^512 larger first (the
+// results there are subnormal or zero); above it `fits` is cleared.
+__device__ __forceinline__ double wide_result(long long T, int e, int khi, int klo, int ke, bool &fits) {
+    double t;
+    asm("cvt.rn.f64.s64 %0, %1;" : "=d"(t) : "l"(T));
+    fits = true;
+    if ((unsigned)(e + ke) >= 2046u) {
+        if (e + ke >= 2046) fits = T == 0;
+        if (e + ke < -500 || T == 0) return 0.0;
+        return t * __hiloint2double(khi + ((e + 512) << 20), klo) * 0x1p-512;
+    }
+    return t * __hiloint2double(khi + (e << 20), klo);
+}
+
+} // namespace f2c

@@ -71,12 +71,12 @@ int f2c_advection_v1(const f2c_grid_v1 *grid, const f2c_fields_v1 *fields, void 
  *   both are bit-identical to the oracle (the reference's strict contract,
  *   compiler/emission/numerical_contract.py:13-15);
  *   F2C_KERNEL_FAST (2): the fast-fp kernel, the counterpart of the
- *   reference's --fast-fp build (compiler/resident/build.py:22): FMA
- *   contraction and an algebraically regrouped form of the same tendencies
- *   (about 80 FP64 operations per point for U, V, W and three scalars, against
- *   126). Results differ from the oracle by rounding only: every field within
- *   1e-12 of its maximum magnitude (measured ~1e-15). In F2C_ADVANCE mode the
- *   time step is folded into the coefficients. */
+ *   reference's --fast-fp build (compiler/resident/build.py:22): an
+ *   algebraically regrouped form of the same tendencies, evaluated in 64-bit
+ *   fixed point at each point's own scale. Results differ from the oracle by
+ *   rounding only: every field within 1e-12 of its maximum magnitude (measured
+ *   ~1e-15). In F2C_ADVANCE mode the time step is folded into the coefficients.
+ */
 enum f2c_kernel_variant { F2C_KERNEL_FACES = 0, F2C_KERNEL_DIRECT = 1, F2C_KERNEL_FAST = 2 };
 int f2c_advection_variant_v1(const f2c_grid_v1 *grid, const f2c_fields_v1 *fields, int variant, void *stream);
 
