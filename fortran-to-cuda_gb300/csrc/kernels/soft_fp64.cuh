@@ -1,35 +1,28 @@
 // Binary64 addition and multiplication on the integer pipes, rounded to
 // nearest-even exactly as IEEE 754-2019 (clauses 4.3.1 and 5.4.1) defines them.
 //
-// GB300 issues FP64 at about two lane operations per clock per SM while its
-// integer pipes (logic, shifts and compares on the ALU pipe, wide multiplies
-// and adds on the FMA pipe) take 64 or more; the advection kernels are bound
-// by the FP64 pipe with the integer pipes nearly idle. Computing part of the
-// additions and multiplications here moves that work to the idle pipes. The
+// GB300 issues FP64 at 1.68 lane operations per clock per SM, while its integer
+// pipes take 64 (shifts, logic, compares and 64-bit additions on the ALU pipe,
+// wide multiplications on the FMA pipe), at the same time: some 38 ALU
+// instructions run in the time of one FP64 operation. The kernels bound by FP64
+// move products (22 ALU instructions) and some additions (50) there. The
 // results are the correctly rounded ones, so they equal the hardware's DADD and
 // DMUL bit for bit: substituting one for the other changes no value.
 //
 // The method is the textbook one (align, add or subtract the significands with
 // a sticky bit jammed into the lowest position, normalise, round to nearest with
-// ties to even; the product's significand as a 106-bit integer), written for the
-// common case only: both operands normal, the result normal. Every other case
-// (zeros, subnormals, infinities, NaN, results that overflow or underflow; all
-// rare in the stencils' fields) is handed to the hardware instruction.
-//
-// The kernels use the product (mul_rn_int). The two additions are kept beside
-// it, checked by the same tests, as the measured alternatives: in the advection
-// kernels, whose integer pipes already carry the products, moving additions
-// off the FP64 pipe made every kernel slower (add_rn_int by about as much time
-// as the DADD it replaces; add_rn_near, about half the integer work, still
-// 4-21 % slower for 6-17 additions per point of the fast-fp kernel).
+// ties to even; the product's significand as a 106-bit integer), written without
+// branches for the common operands: a branch in each operation keeps the
+// compiler from interleaving independent ones. Operands that it does not take
+// (zeros, subnormals, infinities, NaN, the ends of the exponent range; all rare
+// in the stencils' fields) are noted, and the caller does the point again in
+// FP64. Doubles are taken apart as 32-bit words throughout: masking the sign of
+// a double's 64-bit pattern is compiled into an FP64 |x|, two FP64 instructions
+// in an addition meant to save one.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace f2c {
-
-constexpr unsigned long long kSignBit = 0x8000000000000000ull;
-constexpr unsigned long long kFracMask = 0x000FFFFFFFFFFFFFull;
-constexpr unsigned long long kHiddenBit = 0x0010000000000000ull;
 
 // The cases the integer paths leave out, kept out of line: a call stays a
 // branch that only lanes needing it take, where an inline hardware operation
@@ -37,98 +30,121 @@ constexpr unsigned long long kHiddenBit = 0x0010000000000000ull;
 static __device__ __noinline__ double add_rn_hw(double a, double b) { return __dadd_rn(a, b); }
 static __device__ __noinline__ double mul_rn_hw(double a, double b) { return __dmul_rn(a, b); }
 
-// Round a significand with its leading one at bit 63 (bits below bit 0 jammed
-// into bit 0) to 53 bits, nearest-even; the result keeps the hidden bit, or is
-// 2^53 after a carry out of the significand.
-__device__ __forceinline__ unsigned long long round_top53(unsigned long long s) {
-    const unsigned long long m = s >> 11;
-    const unsigned rem = (unsigned)s & 0x7FFu;
-    return m + ((rem > 0x400u || (rem == 0x400u && (m & 1ull))) ? 1ull : 0ull);
+// Words of a 64-bit pattern. On the device they are inline PTX: where the
+// compiler sees a word as a shift of a value whose range it knows, it multiplies
+// 64 x 64 bits instead of 32 x 32 (70 instructions for the product below, not 41).
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ unsigned high_word(unsigned long long x) {
+    unsigned r;
+    asm("{.reg .b32 t; mov.b64 {t, %0}, %1;}" : "=r"(r) : "l"(x));
+    return r;
+}
+__device__ __forceinline__ unsigned low_word(unsigned long long x) {
+    unsigned r;
+    asm("{.reg .b32 t; mov.b64 {%0, t}, %1;}" : "=r"(r) : "l"(x));
+    return r;
+}
+// (h:l + inc * 2^-32) with `top` added to the high word: inc is a carry-in's 32-bit addend below the low word.
+__device__ __forceinline__ unsigned long long add_carry(unsigned h, unsigned l, unsigned below, unsigned inc, unsigned top) {
+    unsigned long long r;
+    asm("{.reg .b32 t, u, v; add.cc.u32 t, %3, %4; addc.cc.u32 u, %2, 0; addc.u32 v, %1, %5; mov.b64 %0, {u, v};}"
+        : "=l"(r) : "r"(h), "r"(l), "r"(below), "r"(inc), "r"(top));
+    return r;
+}
+#else
+inline unsigned high_word(unsigned long long x) { return (unsigned)(x >> 32); }
+inline unsigned low_word(unsigned long long x) { return (unsigned)x; }
+inline unsigned long long add_carry(unsigned h, unsigned l, unsigned below, unsigned inc, unsigned top) {
+    return (((unsigned long long)h << 32) | l) + (((unsigned long long)below + inc) >> 32) + ((unsigned long long)top << 32);
+}
+#endif
+// The high word of hi:lo << n, for n in 1..31.
+__device__ __forceinline__ unsigned shl_high(unsigned hi, unsigned lo, unsigned n) { return (hi << n) | (lo >> (32u - n)); }
+
+// The largest of several operands' distances below 2^-511 as unsigned numbers: from kProductRange on, one of them
+// is outside 2^-511 .. 2^511 (or zero).
+constexpr unsigned kProductRange = 0x3FF00000u;
+
+// a * b, rounded to nearest-even, for operands within 2^-511 .. 2^511 (whose
+// product is normal), without a branch: `range` collects what tells the caller,
+// after any number of products, that one was not (kProductRange), and that they
+// are to be done again in FP64.
+__device__ __forceinline__ double mul_rn_range(double a, double b, unsigned &range) {
+    const unsigned long long ia = (unsigned long long)__double_as_longlong(a);
+    const unsigned long long ib = (unsigned long long)__double_as_longlong(b);
+    const unsigned ahi = high_word(ia), alo = low_word(ia), bhi = high_word(ib), blo = low_word(ib);
+    const unsigned ea = ahi & 0x7FF00000u, eb = bhi & 0x7FF00000u;  // the exponent fields, in place
+    const unsigned ra = ea - 0x20000000u, rb = eb - 0x20000000u, r2 = ra > rb ? ra : rb;
+    range = range > r2 ? range : r2;
+    // significands, a's shifted left by 10: the product's high 64 bits h1:h0 lie in [2^50, 2^52), and the
+    // middle word's sum stays below 2^64
+    const unsigned ah = (shl_high(ahi, alo, 10) & 0x3FFFFFFFu) | 0x40000000u, al = alo << 10;
+    const unsigned bh = (bhi & 0xFFFFFu) | 0x100000u, bl = blo;
+    const unsigned long long low = (unsigned long long)al * bl;
+    const unsigned long long mid = (unsigned long long)ah * bl + (unsigned long long)al * bh + high_word(low);
+    const unsigned long long high = (unsigned long long)ah * bh + high_word(mid);
+    const unsigned l0 = low_word(low);
+    unsigned l1 = low_word(mid) | (l0 < 1u ? l0 : 1u);  // the word below, the lowest one jammed into it
+    unsigned h1 = high_word(high), h0 = low_word(high);
+    const unsigned z = 2u - (h1 >> 19);  // left shift that brings the leading one to bit 52
+    h1 = shl_high(h1, h0, z);
+    h0 = shl_high(h0, l1, z);
+    l1 <<= z;
+    // rounds up when the word below is over half, or half with h0 odd; the leading one adds to the exponent field
+    const unsigned long long r = add_carry(h1, h0, l1, 0x7FFFFFFFu + (h0 & 1u), ea + eb - (z << 20) - (1022u << 20));
+    return __longlong_as_double((long long)(r | ((unsigned long long)((ahi ^ bhi) & 0x80000000u) << 32)));
 }
 
-// a + b, rounded to nearest-even.
+// What add_rn_range collects over any number of additions.
+struct SumRange {
+    unsigned apart = 0, end = 0;  // largest exponent difference, and distance below 2^-959 (unsigned)
+    int top = 63;                 // lowest leading bit of a sum (-1: zero)
+    __device__ __forceinline__ bool left() const { return apart > 0x01F00000u || end > 0x77000000u || top < 0; }
+};
+
+// a + b, rounded to nearest-even, without a branch, for operands between 2^-959
+// and 2^945 at most 2^31 apart, with a sum that is not zero; `range` collects
+// what tells the caller that one was not so, and that the sums are to be done
+// again in FP64.
+__device__ __forceinline__ double add_rn_range(double a, double b, SumRange &range) {
+    const unsigned long long ia = (unsigned long long)__double_as_longlong(a);
+    const unsigned long long ib = (unsigned long long)__double_as_longlong(b);
+    const unsigned ahi = high_word(ia), alo = low_word(ia), bhi = high_word(ib), blo = low_word(ib);
+    // the larger magnitude first (compared as words: a sign cleared in a double's 64 bits becomes an FP64 |x|)
+    const unsigned ha = ahi & 0x7FFFFFFFu, hb = bhi & 0x7FFFFFFFu;
+    const bool swap = (((unsigned long long)ha << 32) | alo) < (((unsigned long long)hb << 32) | blo);
+    const unsigned xh = swap ? bhi : ahi, xl = swap ? blo : alo, yh = swap ? ahi : bhi, yl = swap ? alo : blo;
+    const unsigned xe = xh & 0x7FF00000u, ye = yh & 0x7FF00000u, apart = xe - ye, end = ye - 0x04000000u;
+    range.apart = range.apart > apart ? range.apart : apart;
+    range.end = range.end > end ? range.end : end;
+    // significands with the leading bit at 61; the smaller one, a bit higher, shifted right by one and the
+    // exponents' difference as a product by 2^(31 - difference), what that drops jammed into the lowest bit
+    const unsigned long long x = ((unsigned long long)((shl_high(xh, xl, 9) & 0x1FFFFFFFu) | 0x20000000u) << 32) | (xl << 9);
+    const unsigned sh = (shl_high(yh, yl, 10) & 0x3FFFFFFFu) | 0x40000000u, sl = yl << 10, f = 0x80000000u >> ((apart >> 20) & 31u);
+    const unsigned long long low = (unsigned long long)sl * f, high = (unsigned long long)sh * f + high_word(low);
+    const unsigned lost = low_word(low), less = (unsigned)((int)(xh ^ yh) >> 31);
+    const unsigned long long y = ((unsigned long long)(high_word(high) ^ less) << 32) | ((low_word(high) | (lost < 1u ? lost : 1u)) ^ less);
+    const unsigned long long s = x + y - (unsigned long long)(long long)(int)less;
+    const int top = 63 - __clzll((long long)s);
+    range.top = range.top < top ? range.top : top;
+    const unsigned long long n = s << ((62 - top) & 63);
+    const unsigned h0 = low_word(n);
+    const unsigned long long r = (n + (0x1FFu + ((h0 >> 10) & 1u))) >> 10;
+    return __longlong_as_double((long long)(r + ((unsigned long long)((xh & 0xFFF00000u) + ((unsigned)(top - 62) << 20)) << 32)));
+}
+
+// The same with operands outside the range going to the hardware operation.
 __device__ __forceinline__ double add_rn_int(double a, double b) {
-    const unsigned long long ia = (unsigned long long)__double_as_longlong(a);
-    const unsigned long long ib = (unsigned long long)__double_as_longlong(b);
-    const unsigned long long ma = ia & ~kSignBit, mb = ib & ~kSignBit;
-    const bool swap = ma < mb;
-    const unsigned long long x = swap ? ib : ia;  // the operand of larger magnitude: the result's sign
-    const unsigned long long mx = swap ? mb : ma, my = swap ? ma : mb;
-    const int ex = (int)(mx >> 52), ey = (int)(my >> 52);
-    if (ey == 0 || ex > 0x7FC) return add_rn_hw(a, b);
-    // significands with the hidden bit at bit 62 (ten spare low bits)
-    const unsigned long long fx = ((mx & kFracMask) | kHiddenBit) << 10;
-    unsigned long long fy = ((my & kFracMask) | kHiddenBit) << 10;
-    const unsigned d = (unsigned)min(ex - ey, 63);
-    const unsigned long long kept = fy >> d;
-    fy = kept | (unsigned long long)((kept << d) != fy);  // jam the bits shifted out into bit 0
-    const bool sub = (long long)(ia ^ ib) < 0;
-    unsigned long long s = sub ? fx - fy : fx + fy;
-    if (s == 0) return 0.0;  // x + (-x) is +0 when rounding to nearest
-    const int lz = __clzll((long long)s);
-    s <<= lz;                 // leading one at bit 63
-    const int e = ex + 1 - lz;  // biased exponent of the result
-    if (e < 1) return add_rn_hw(a, b);
-    const unsigned long long m = round_top53(s);
-    // m carries the hidden bit (or 2^53 after a rounding carry), so adding it to (e - 1) << 52 also
-    // carries into the exponent when rounding overflowed the significand
-    return __longlong_as_double((long long)((x & kSignBit) | (((unsigned long long)(e - 1) << 52) + m)));
+    SumRange range;
+    const double r = add_rn_range(a, b, range);
+    return range.left() ? add_rn_hw(a, b) : r;
 }
-
-// a + b, rounded to nearest-even, for operands whose exponents differ by at
-// most 9 (the sum of neighbouring values of a smooth field): aligned to the
-// smaller exponent the significands add exactly in 64 bits, so the only
-// rounding is the final one, which needs no sticky bit. About half the
-// integer work of add_rn_int; other operands go to the hardware addition.
-__device__ __forceinline__ double add_rn_near(double a, double b) {
-    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-    const int ea = (int)((unsigned long long)ia >> 52) & 0x7FF, eb = (int)((unsigned long long)ib >> 52) & 0x7FF;
-    const int d = ea - eb;
-    if ((unsigned)(ea - 1) >= 0x7FCu || (unsigned)(eb - 1) >= 0x7FCu || (unsigned)(d + 9) > 18u) return add_rn_hw(a, b);
-    long long ma = (ia & (long long)kFracMask) | (long long)kHiddenBit;
-    long long mb = (ib & (long long)kFracMask) | (long long)kHiddenBit;
-    ma <<= (d > 0 ? d : 0);  // below 2^62
-    mb <<= (d < 0 ? -d : 0);
-    const int e0 = d > 0 ? eb : ea;
-    const long long s = (ia < 0 ? -ma : ma) + (ib < 0 ? -mb : mb);  // exact, |s| < 2^63
-    const unsigned long long mag = (unsigned long long)(s < 0 ? -s : s);
-    if (mag == 0) return 0.0;  // x + (-x) is +0 when rounding to nearest
-    const int sh = 11 - __clzll((long long)mag);  // bits below the 53 the result keeps
-    unsigned long long m;
-    if (sh > 0) {
-        const unsigned long long half = 1ull << (sh - 1), rest = mag & ((half << 1) - 1);
-        m = (mag + half) >> sh;
-        if (rest == half) m &= ~1ull;  // a tie goes to the even significand
-    } else {
-        m = mag << (-sh);
-    }
-    const int e = e0 + sh;  // biased exponent of the result
-    if (e < 1) return add_rn_hw(a, b);
-    return __longlong_as_double((long long)((s < 0 ? kSignBit : 0ull) | (((unsigned long long)(e - 1) << 52) + m)));
-}
-
-// a * b, rounded to nearest-even.
+// add_rn_int for operands of nearby exponents, which need no other path.
+__device__ __forceinline__ double add_rn_near(double a, double b) { return add_rn_int(a, b); }
 __device__ __forceinline__ double mul_rn_int(double a, double b) {
-    const unsigned long long ia = (unsigned long long)__double_as_longlong(a);
-    const unsigned long long ib = (unsigned long long)__double_as_longlong(b);
-    const int ea = (int)((ia >> 52) & 0x7FF), eb = (int)((ib >> 52) & 0x7FF);
-    int e = ea + eb - 1023;  // biased exponent when the significand product is below 2
-    if (ea == 0 || eb == 0 || ea == 0x7FF || eb == 0x7FF || e < 1 || e > 0x7FC) return mul_rn_hw(a, b);
-    const unsigned long long fa = (ia & kFracMask) | kHiddenBit, fb = (ib & kFracMask) | kHiddenBit;
-    // the 106-bit product hi * 2^64 + lo from 32-bit pieces (the high pieces are below 2^21)
-    const unsigned al = (unsigned)fa, ah = (unsigned)(fa >> 32), bl = (unsigned)fb, bh = (unsigned)(fb >> 32);
-    const unsigned long long ll = (unsigned long long)al * bl;
-    const unsigned long long mid = (unsigned long long)al * bh + (unsigned long long)ah * bl;  // below 2^54
-    const unsigned long long lo = ll + (mid << 32);
-    const unsigned long long hi = (unsigned long long)ah * bh + (mid >> 32) + (lo < ll ? 1ull : 0ull);
-    // top 64 bits of the product (it lies in [2^104, 2^106)), the 42 bits below jammed into bit 0
-    unsigned long long t = (hi << 22) | (lo >> 42) | ((lo & ((1ull << 42) - 1)) != 0 ? 1ull : 0ull);
-    const int lz = (int)(~t >> 63);  // 0 when the product reached 2^105
-    t <<= lz;
-    e += 1 - lz;
-    const unsigned long long m = round_top53(t);
-    return __longlong_as_double(
-        (long long)(((ia ^ ib) & kSignBit) | (((unsigned long long)(e - 1) << 52) + m)));
+    unsigned range = 0;
+    const double r = mul_rn_range(a, b, range);
+    return range >= kProductRange ? mul_rn_hw(a, b) : r;
 }
 
 } // namespace f2c

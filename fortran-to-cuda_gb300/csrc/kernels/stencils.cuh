@@ -15,9 +15,12 @@
 
 #include "soft_fp64.cuh"
 
-// The products below run on the integer pipes (mul_rn_int: the correctly
-// rounded product, the same bits as DMUL), leaving the FP64 pipe, which bounds
-// these stencils, to the additions.
+// FP64 additions bound these stencils (1.68 lanes a clock per SM), so the
+// products and as many additions as balance the two run on the integer pipes
+// (soft_fp64.cuh; the correctly rounded results, the same bits), without
+// branches: a point whose operands they cannot take is done again in FP64. The
+// additions moved are ones along y: a zero of the west or east boundary would
+// send a warp of every row that way, one of the others only the outer rows'.
 namespace f2c {
 
 // x * 2^e for an exact power-of-two factor, on the integer pipe when the
@@ -36,6 +39,16 @@ __device__ __forceinline__ double scale_pow2(double x, int e, double factor) {
     return scale_by(x, factor);
 }
 
+// IEEE negation on the integer pipe (a plain -x here becomes an FP64 addition).
+__device__ __forceinline__ double sign_flipped(double x) {
+    unsigned long long r;
+    asm("xor.b64 %0, %1, 0x8000000000000000;" : "=l"(r) : "l"((unsigned long long)__double_as_longlong(x)));
+    return __longlong_as_double((long long)r);
+}
+
+// The division where dx*dx is no power of two, out of line (inline it is evaluated for every point).
+static __device__ __noinline__ double divide(double x, double y) { return x / y; }
+
 struct DiffusionArgs {
     const double *a;
     double *b;
@@ -49,6 +62,9 @@ struct DiffusionArgs {
 
 constexpr int kDiffBX = 32, kDiffBY = 8, kDiffKZ = 32;
 
+// 384^3: 0.59 ms with two of the seven additions on the integer pipes (0.79 with
+// none, 0.70 with one, 0.69 with three: an addition there takes 50 ALU
+// instructions, an FP64 one the time of 38).
 static __global__ void __launch_bounds__(kDiffBX *kDiffBY) diffusion7_kernel(const DiffusionArgs p) {
     const int i = blockIdx.x * kDiffBX + threadIdx.x;
     const int j = blockIdx.y * kDiffBY + threadIdx.y;
@@ -59,12 +75,23 @@ static __global__ void __launch_bounds__(kDiffBX *kDiffBY) diffusion7_kernel(con
     const long long sx = p.sx, plane = p.plane;
     long long q = (long long)(i + p.h) + sx * (long long)(j + p.h) + plane * (long long)(k0 + p.h);
     double below = __ldg(A + q - plane), centre = __ldg(A + q);
+    // an exact scaling commutes with the product after it (its operand within 2^-511 .. 2^511, the scale within 2^-256 .. 2^256)
+    const bool folded = p.dx2_pow2 && p.dx2_exp >= -256 && p.dx2_exp <= 256;
+    const double factor = folded ? scale_pow2(p.dtnu, -p.dx2_exp, 1.0 / p.dx2) : p.dtnu;
     for (int k = k0; k < k1; ++k, q += plane) {
+        const double west = __ldg(A + q - 1), east = __ldg(A + q + 1), south = __ldg(A + q - sx), north = __ldg(A + q + sx);
         const double above = __ldg(A + q + plane);
-        const double sum = __ldg(A + q - 1) + __ldg(A + q + 1) + __ldg(A + q - sx) + __ldg(A + q + sx) + below + above;
-        const double num = sum - mul_rn_int(6.0, centre);
-        const double lap = p.dx2_pow2 ? scale_pow2(num, -p.dx2_exp, 1.0 / p.dx2) : num / p.dx2;
-        p.b[q] = centre + mul_rn_int(p.dtnu, lap);
+        unsigned range = 0;
+        SumRange sums;
+        const double first = add_rn_range(add_rn_range(west + east, south, sums), north, sums);
+        const double num = (first + below + above) - mul_rn_range(6.0, centre, range);
+        const double lap = folded ? num : divide(num, p.dx2);
+        double r = centre + mul_rn_range(factor, lap, range);
+        if (range >= kProductRange || sums.left()) {
+            const double n = add_rn_hw(add_rn_hw(add_rn_hw(west, east), south), north) + below + above - mul_rn_hw(6.0, centre);
+            r = centre + mul_rn_hw(p.dtnu, p.dx2_pow2 ? scale_pow2(n, -p.dx2_exp, 1.0 / p.dx2) : n / p.dx2);
+        }
+        p.b[q] = r;
         below = centre;
         centre = above;
     }
@@ -79,6 +106,8 @@ struct JacobiArgs {
 
 constexpr int kJacBX = 64, kJacBY = 4, kJacJY = 8;  // each thread does kJacJY rows
 
+// 8192^2: 0.27 ms with one of the three additions on the integer pipes (0.39 with
+// none, 0.34 with three in two rows).
 static __global__ void __launch_bounds__(kJacBX *kJacBY) jacobi5_kernel(const JacobiArgs p) {
     const int i = blockIdx.x * kJacBX + threadIdx.x;
     const int j0 = (blockIdx.y * kJacBY + threadIdx.y) * kJacJY;
@@ -90,9 +119,12 @@ static __global__ void __launch_bounds__(kJacBX *kJacBY) jacobi5_kernel(const Ja
     double south = j0 < p.ny ? __ldg(U + q - sx) : 0.0;
     double centre = j0 < p.ny ? __ldg(U + q) : 0.0;
     for (int j = j0; j < j1; ++j, q += sx) {
-        const double north = __ldg(U + q + sx);
-        const double sum = __ldg(U + q - 1) + __ldg(U + q + 1) + south + north;
-        p.v[q] = scale_pow2(sum, -2, 0.25);
+        const double north = __ldg(U + q + sx), west = __ldg(U + q - 1), east = __ldg(U + q + 1);
+        SumRange sums;
+        const double across = west + east;
+        double three = add_rn_range(across, south, sums);
+        if (sums.left()) three = add_rn_hw(across, south);
+        p.v[q] = scale_pow2(three + north, -2, 0.25);
         south = centre;
         centre = north;
     }
@@ -105,24 +137,53 @@ struct YeeArgs {
     long long sx;
 };
 
-constexpr int kYeeBX = 64, kYeeBY = 4;
+// 4096^2: 0.245 ms a step with one addition of four on the integer pipes in each kernel (0.14 + 0.11; 0.28 with none).
+constexpr int kYeeBX = 64, kYeeBY = 4, kYeeJY = 2;  // each thread does kYeeJY rows
 
 static __global__ void __launch_bounds__(kYeeBX *kYeeBY) yee_h_kernel(const YeeArgs p) {
     const int i = blockIdx.x * kYeeBX + threadIdx.x;
-    const int j = blockIdx.y * kYeeBY + threadIdx.y;
-    if (i >= p.nx || j >= p.ny) return;
-    const long long q = (long long)(i + p.h) + p.sx * (long long)(j + p.h);
-    const double e = __ldg(p.ez + q);
-    p.hx[q] = p.hx[q] - mul_rn_int(p.ch, __ldg(p.ez + q + p.sx) - e);
-    p.hy[q] = p.hy[q] + mul_rn_int(p.ch, __ldg(p.ez + q + 1) - e);
+    const int j0 = (blockIdx.y * kYeeBY + threadIdx.y) * kYeeJY;
+    if (i >= p.nx || j0 >= p.ny) return;
+    long long q = (long long)(i + p.h) + p.sx * (long long)(j0 + p.h);
+    const int j1 = min(j0 + kYeeJY, p.ny);
+    double e = __ldg(p.ez + q);
+#pragma unroll
+    for (int j = j0; j < j0 + kYeeJY; ++j, q += p.sx) {
+        if (j >= j1) return;
+        const double north = __ldg(p.ez + q + p.sx), east = __ldg(p.ez + q + 1);
+        const double hx = p.hx[q], hy = p.hy[q];
+        unsigned range = 0;
+        SumRange sums;
+        double x = hx - mul_rn_range(p.ch, add_rn_range(north, sign_flipped(e), sums), range);
+        double y = hy + mul_rn_range(p.ch, east - e, range);
+        if (range >= kProductRange || sums.left()) {
+            x = hx - mul_rn_hw(p.ch, north - e);
+            y = hy + mul_rn_hw(p.ch, east - e);
+        }
+        p.hx[q] = x;
+        p.hy[q] = y;
+        e = north;
+    }
 }
 
 static __global__ void __launch_bounds__(kYeeBX *kYeeBY) yee_e_kernel(const YeeArgs p) {
     const int i = blockIdx.x * kYeeBX + threadIdx.x;
-    const int j = blockIdx.y * kYeeBY + threadIdx.y;
-    if (i >= p.nx || j >= p.ny) return;
-    const long long q = (long long)(i + p.h) + p.sx * (long long)(j + p.h);
-    p.ez[q] = p.ez[q] + mul_rn_int(p.ce, (__ldg(p.hy + q) - __ldg(p.hy + q - 1)) - (__ldg(p.hx + q) - __ldg(p.hx + q - p.sx)));
+    const int j0 = (blockIdx.y * kYeeBY + threadIdx.y) * kYeeJY;
+    if (i >= p.nx || j0 >= p.ny) return;
+    long long q = (long long)(i + p.h) + p.sx * (long long)(j0 + p.h);
+    const int j1 = min(j0 + kYeeJY, p.ny);
+    double south = __ldg(p.hx + q - p.sx);
+#pragma unroll
+    for (int j = j0; j < j0 + kYeeJY; ++j, q += p.sx) {
+        if (j >= j1) return;
+        const double ez = p.ez[q], hy = __ldg(p.hy + q), west = __ldg(p.hy + q - 1), hx = __ldg(p.hx + q);
+        unsigned range = 0;
+        SumRange sums;
+        double e = ez + mul_rn_range(p.ce, (hy - west) - add_rn_range(hx, sign_flipped(south), sums), range);
+        if (range >= kProductRange || sums.left()) e = ez + mul_rn_hw(p.ce, (hy - west) - (hx - south));
+        p.ez[q] = e;
+        south = hx;
+    }
 }
 
 inline dim3 diffusion_grid(const DiffusionArgs &p) {
@@ -131,7 +192,7 @@ inline dim3 diffusion_grid(const DiffusionArgs &p) {
 inline dim3 jacobi_grid(const JacobiArgs &p) {
     return dim3((p.nx + kJacBX - 1) / kJacBX, (p.ny + kJacBY * kJacJY - 1) / (kJacBY * kJacJY), 1);
 }
-inline dim3 yee_grid(const YeeArgs &p) { return dim3((p.nx + kYeeBX - 1) / kYeeBX, (p.ny + kYeeBY - 1) / kYeeBY, 1); }
+inline dim3 yee_grid(const YeeArgs &p) { return dim3((p.nx + kYeeBX - 1) / kYeeBX, (p.ny + kYeeBY * kYeeJY - 1) / (kYeeBY * kYeeJY), 1); }
 
 // Exponent e with x == 2^e exactly, or a flag that x is not a power of two.
 inline bool power_of_two(double x, int *e) {
