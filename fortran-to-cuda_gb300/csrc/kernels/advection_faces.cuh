@@ -20,17 +20,20 @@
 //    rounded subnormal case handled in integer arithmetic as well).
 //
 // Every other operation follows the reference grouping (advection_point.cuh),
-// so results are bit-identical to the oracle. The advective-form products and
-// the second product of each face flux are computed on the integer pipes (pmul
-// below, rounded exactly as DMUL): 27 of the 48 products per point with three
-// scalars. That split balances the pipes; measured at 512 x 512 x 128 with
-// three scalars (two CTAs per SM): 8.74 ms with every product a DMUL, 8.17 ms with all 48 on the
-// integer pipes (the FP64 pipe then waits on the longer integer chains, 62 %
-// busy), 7.33 ms with these 27 (7.69 with the advective ones alone, 7.46 with
-// both flux products as well). Operation count per point:
-// U, V, W: 9 face sums + 18 flux products + 15 flux differences + 48
-// advective-form operations = 90; scalars: 3 shared coefficient products +
-// 11 per scalar.
+// so results are bit-identical to the oracle. All products and the advective
+// forms' differences are computed on the integer pipes (soft_fp64.cuh, rounded
+// exactly as DMUL and DADD), without branches: the operands that those do not
+// take (zeros at the walls among them) have the thread do its half of the level
+// again in FP64. Operation count per point: U, V, W: 9 face sums + 18 flux
+// products + 15 flux differences + 48 advective-form operations = 90; scalars: 3
+// shared coefficient products + 11 per scalar. Of the 126 with three scalars 69
+// are left to the FP64 pipe. Measured at 512 x 512 x 128 without and with three
+// scalars: 4.83 and 7.41 ms with 27 products on the integer pipes, each with a
+// branch; 4.30 and 6.47 with all 48, without; 4.12 and 6.40 with the nine
+// differences as well; 4.37 and 6.99 with the nine face sums instead, 4.72 and
+// 6.77 with the differences and the advecting sums (registers: 72 a thread). On
+// the sine-mode fields with a Gaussian tracer: 3.95 and 6.02 ms (7.13 before;
+// 7.01 with one range for momentum and scalars, whose tails then cost both).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -42,12 +45,6 @@
 
 namespace f2c {
 
-// Products on the integer pipes (soft_fp64.cuh): bit-identical to DMUL, they
-// take multiplications off the FP64 pipe that bounds these kernels. Additions
-// stay on the FP64 pipe: an integer addition costs about as much time on the
-// ALU pipe as it saves on the FP64 one (measured slower).
-__device__ __forceinline__ double pmul(double a, double b) { return mul_rn_int(a, b); }
-
 constexpr int kFaceTX = 32;       // points per tile along x (one warp)
 constexpr int kFaceTY = 8;        // compute warps per tile (points along y)
 constexpr int kFaceKZ = 32;       // levels per z-chunk
@@ -56,9 +53,8 @@ constexpr int kFaceThreads = kFaceTX * (kFaceTY + 1);
 // warps hide the FP64, integer and shared-memory latencies. What made room for
 // the third CTA is phase B reading the point's own fluxes back from the shared
 // rows and its values again from L1 (ldg_again) instead of holding them in
-// registers across the barrier. Measured at 512 x 512 x 128 with three
-// scalars: 7.33 ms at two CTAs before that change (8.04 at three, with twice
-// the spills), 7.26 ms at two and 7.11 at three after it.
+// registers across the barrier. 512 x 512 x 128 with three scalars: 6.40 ms, at
+// two CTAs 6.41; without scalars 4.13 and 4.44.
 constexpr int kFaceCtasPerSM = 3;
 
 // Exact x * 0.5 without the FP64 pipe: for normal x the exponent field drops by
@@ -180,6 +176,15 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
             U0 = LD(U, p, 0, 0, 0); Ue = LD(U, p, 1, 0, 0); Un = LD(U, p, 0, 1, 0); Up = LD(U, p, 0, 0, 1);
             V0 = LD(V, p, 0, 0, 0); Ve = LD(V, p, 1, 0, 0); Vn = LD(V, p, 0, 1, 0); Vp = LD(V, p, 0, 0, 1);
             W0 = LD(W, p, 0, 0, 0); We = LD(W, p, 1, 0, 0); Wn = LD(W, p, 0, 1, 0); Wp = LD(W, p, 0, 0, 1);
+            double se[NS > 0 ? NS : 1], sn[NS > 0 ? NS : 1], st[NS > 0 ? NS : 1];
+#pragma unroll
+            for (int n = 0; n < NS; ++n) {
+                const double *__restrict__ S = a.s[n];
+                S0[n] = LD(S, p, 0, 0, 0);
+                se[n] = LD(S, p, 1, 0, 0);
+                sn[n] = LD(S, p, 0, 1, 0);
+                st[n] = LD(S, p, 0, 0, 1);
+            }
             if (DO_U) sUx = Ue + U0;
             if (DO_U || DO_V) sVx = Ve + V0;
             if (DO_U || DO_W) sWx = We + W0;
@@ -189,30 +194,47 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
             if (DO_U || DO_W) sUz = Up + U0;
             if (DO_V || DO_W) sVz = Vp + V0;
             if (DO_W) sWz = Wp + W0;
-            if (DO_U) {
-                FUx = pmul(c.Ax * sUx, sUx);
-                FUy = pmul(c.Ay * sUy, sVx);
-                FUz = pmul(c.Az * sUz, sWx);
-            }
-            if (DO_V) {
-                FVx = pmul(c.Ax * sVx, sUy);
-                FVy = pmul(c.Ay * sVy, sVy);
-                FVz = pmul(c.Az * sVz, sWy);
-            }
-            if (DO_W) {
-                FWx = pmul(c.Ax * sWx, sUz);
-                FWy = pmul(c.Ay * sWy, sVz);
-                FWz = pmul(c.Az * sWz, sWz);
-            }
+            auto fluxes = [&](auto mul) {
+                if (DO_U) {
+                    FUx = mul(mul(c.Ax, sUx), sUx);
+                    FUy = mul(mul(c.Ay, sUy), sVx);
+                    FUz = mul(mul(c.Az, sUz), sWx);
+                }
+                if (DO_V) {
+                    FVx = mul(mul(c.Ax, sVx), sUy);
+                    FVy = mul(mul(c.Ay, sVy), sVy);
+                    FVz = mul(mul(c.Az, sVz), sWy);
+                }
+                if (DO_W) {
+                    FWx = mul(mul(c.Ax, sWx), sUz);
+                    FWy = mul(mul(c.Ay, sWy), sVz);
+                    FWz = mul(mul(c.Az, sWz), sWz);
+                }
+            };
+            ProductRange<false> range;
+            fluxes([&](double x, double y) { return mul_rn_range(x, y, range); });
+            if (range.left()) fluxes([](double x, double y) { return mul_rn_hw(x, y); });
             if (NS > 0) {
-                const double SxU = c.Sx * U0, SyV = c.Sy * V0, SzW = c.Sz * W0;
+                // a scalar's own range: a tracer's zeros and tails (which WIDE takes further down) cost its own products only
+                ProductRange<true> shared;
+                double SxU = mul_rn_range(c.Sx, U0, shared), SyV = mul_rn_range(c.Sy, V0, shared), SzW = mul_rn_range(c.Sz, W0, shared);
+                if (shared.left()) {
+                    SxU = mul_rn_hw(c.Sx, U0);
+                    SyV = mul_rn_hw(c.Sy, V0);
+                    SzW = mul_rn_hw(c.Sz, W0);
+                }
 #pragma unroll
                 for (int n = 0; n < NS; ++n) {
-                    const double *__restrict__ S = a.s[n];
-                    S0[n] = LD(S, p, 0, 0, 0);
-                    fe[n] = SxU * (LD(S, p, 1, 0, 0) + S0[n]);
-                    fn[n] = SyV * (LD(S, p, 0, 1, 0) + S0[n]);
-                    ft[n] = SzW * (LD(S, p, 0, 0, 1) + S0[n]);
+                    ProductRange<true> own;
+                    const double e = se[n] + S0[n], f = sn[n] + S0[n], g = st[n] + S0[n];
+                    fe[n] = mul_rn_range(SxU, e, own);
+                    fn[n] = mul_rn_range(SyV, f, own);
+                    ft[n] = mul_rn_range(SzW, g, own);
+                    if (own.left()) {
+                        fe[n] = mul_rn_hw(SxU, e);
+                        fn[n] = mul_rn_hw(SyV, f);
+                        ft[n] = mul_rn_hw(SzW, g);
+                    }
                 }
             }
             const int xo = warp * (kFaceTX + 1) + lane + 1;
@@ -296,28 +318,43 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
             const double Uw = LD(U, p, -1, 0, 0), Us = LD(U, p, 0, -1, 0), Um = LD(U, p, 0, 0, -1);
             const double Vw = LD(V, p, -1, 0, 0), Vs = LD(V, p, 0, -1, 0), Vm = LD(V, p, 0, 0, -1);
             const double Ww = LD(W, p, -1, 0, 0), Ws = LD(W, p, 0, -1, 0), Wm = LD(W, p, 0, 0, -1);
+            double aU[3] = {0, 0, 0}, aV[3] = {0, 0, 0}, aW[3] = {0, 0, 0};  // the advective forms' terms
+            auto advective = [&](auto mul, auto sub) {
+                if (DO_U) {
+                    aU[0] = mul(mul(c.Bux, sub(LDA(U, 1, 0, 0), Uw)), Uc);
+                    aU[1] = mul(mul(c.Buy, sub(LDA(U, 0, 1, 0), Us)), (sVx + Vs) + LD(V, p, 1, -1, 0));
+                    aU[2] = mul(mul(c.Buz, sub(LDA(U, 0, 0, 1), Um)), (sWx + Wm) + LD(W, p, 1, 0, -1));
+                }
+                if (DO_V) {
+                    aV[0] = mul(mul(c.Bvx, sub(LDA(V, 1, 0, 0), Vw)), (sUy + Uw) + LD(U, p, -1, 1, 0));
+                    aV[1] = mul(mul(c.Bvy, sub(LDA(V, 0, 1, 0), Vs)), Vc);
+                    aV[2] = mul(mul(c.Bvz, sub(LDA(V, 0, 0, 1), Vm)), (sWy + Wm) + LD(W, p, 0, 1, -1));
+                }
+                if (DO_W) {
+                    aW[0] = mul(mul(c.Bwx, sub(LDA(W, 1, 0, 0), Ww)), (sUz + Uw) + LD(U, p, -1, 0, 1));
+                    aW[1] = mul(mul(c.Bwy, sub(LDA(W, 0, 1, 0), Ws)), (sVz + Vs) + LD(V, p, 0, -1, 1));
+                    aW[2] = mul(mul(c.Bwz, sub(LDA(W, 0, 0, 1), Wm)), Wc);
+                }
+            };
+            ProductRange<false> range;
+            SumRange sums;
+            advective([&](double x, double y) { return mul_rn_range(x, y, range); },
+                      [&](double x, double y) { return add_rn_range(x, opaque_negate(y), sums); });
+            if (range.left() || sums.left())
+                advective([](double x, double y) { return mul_rn_hw(x, y); }, [](double x, double y) { return x - y; });
             if (DO_U) {
                 const double r = opaque_negate(((xf[0 * Smem::XF + xo] - xf[0 * Smem::XF + xw]) + (yf[0 * Smem::YF + yo] - yf[0 * Smem::YF + ys])) + (FUz - FUzb));
-                const double Vadv = (sVx + Vs) + LD(V, p, 1, -1, 0);
-                const double Wadv = (sWx + Wm) + LD(W, p, 1, 0, -1);
-                const double adv = (pmul(pmul(c.Bux, LDA(U, 1, 0, 0) - Uw), Uc) + pmul(pmul(c.Buy, LDA(U, 0, 1, 0) - Us), Vadv)) + pmul(pmul(c.Buz, LDA(U, 0, 0, 1) - Um), Wadv);
-                if (a.out[0]) store_point_t<FILL>(a.out[0], U, p, exact_half(r - adv), a, 0, i, j, k);
+                if (a.out[0]) store_point_t<FILL>(a.out[0], U, p, exact_half(r - ((aU[0] + aU[1]) + aU[2])), a, 0, i, j, k);
                 FUzb = FUz;
             }
             if (DO_V) {
                 const double r = opaque_negate(((yf[1 * Smem::YF + yo] - yf[1 * Smem::YF + ys]) + (xf[1 * Smem::XF + xo] - xf[1 * Smem::XF + xw])) + (FVz - FVzb));
-                const double Uadv = (sUy + Uw) + LD(U, p, -1, 1, 0);
-                const double Wadv = (sWy + Wm) + LD(W, p, 0, 1, -1);
-                const double adv = (pmul(pmul(c.Bvx, LDA(V, 1, 0, 0) - Vw), Uadv) + pmul(pmul(c.Bvy, LDA(V, 0, 1, 0) - Vs), Vc)) + pmul(pmul(c.Bvz, LDA(V, 0, 0, 1) - Vm), Wadv);
-                if (a.out[1]) store_point_t<FILL>(a.out[1], V, p, exact_half(r - adv), a, 0, i, j, k);
+                if (a.out[1]) store_point_t<FILL>(a.out[1], V, p, exact_half(r - ((aV[0] + aV[1]) + aV[2])), a, 0, i, j, k);
                 FVzb = FVz;
             }
             if (DO_W) {
                 const double r = opaque_negate(((FWz - FWzb) + (yf[2 * Smem::YF + yo] - yf[2 * Smem::YF + ys])) + (xf[2 * Smem::XF + xo] - xf[2 * Smem::XF + xw]));
-                const double Uadv = (sUz + Uw) + LD(U, p, -1, 0, 1);
-                const double Vadv = (sVz + Vs) + LD(V, p, 0, -1, 1);
-                const double adv = (pmul(pmul(c.Bwx, LDA(W, 1, 0, 0) - Ww), Uadv) + pmul(pmul(c.Bwy, LDA(W, 0, 1, 0) - Ws), Vadv)) + pmul(pmul(c.Bwz, LDA(W, 0, 0, 1) - Wm), Wc);
-                if (a.out[2]) store_point_t<FILL>(a.out[2], W, p, exact_half(r - adv), a, 1, i, j, k);
+                if (a.out[2]) store_point_t<FILL>(a.out[2], W, p, exact_half(r - ((aW[0] + aW[1]) + aW[2])), a, 1, i, j, k);
                 FWzb = FWz;
             }
 #pragma unroll
@@ -340,18 +377,26 @@ __global__ void __launch_bounds__(kFaceThreads, kFaceCtasPerSM) advection_faces_
     faces_tile<NS, MASK>(a, blockIdx.x, blockIdx.y, k0, min(k0 + a.kz, a.nz), smem);
 }
 
-// Depth of the z-chunks of one launch: deep (kFaceKZ) when the grid has work
-// for several waves of CTAs, shallower for small grids so that at least four
-// CTAs per SM are available (down to two levels, where the per-chunk prologue
-// stays a small fraction of the work).
+// Depth of the z-chunks of one launch: the one with the least time on the SM
+// with the most CTAs, whose levels (and about half a level for a chunk's start)
+// the FP64 pipe takes one after another; one CTA more is counted because the
+// last ones have the SM to themselves and wait on latencies. 161 x 203 x 47 with
+// a scalar: 4 levels, 0.31 ms (13, as four CTAs per SM would have, 0.35);
+// 64^3, U alone: one level, 18.6 us (2: 20.5).
 inline int chunk_depth(int nx, int ny, int nz) {
-    const int sms = current_sm_count();
+    const long long sms = current_sm_count();
     const long long tiles = (long long)((nx + kFaceTX - 1) / kFaceTX) * ((ny + kFaceTY - 1) / kFaceTY);
-    const long long want = 4LL * sms;
-    long long kz = (tiles * nz + want - 1) / want;
-    if (kz > kFaceKZ) kz = kFaceKZ;
-    if (kz < 2) kz = 2;
-    return (int)kz;
+    long long best = -1;
+    int depth = 1;
+    for (int kz = 1; kz <= kFaceKZ && kz <= nz; ++kz) {
+        const long long ctas = tiles * ((nz + kz - 1) / kz);
+        const long long cost = ((ctas + sms - 1) / sms + 1) * (2 * kz + 1);
+        if (best < 0 || cost <= best) {
+            best = cost;
+            depth = kz;
+        }
+    }
+    return depth;
 }
 
 template <int NS, int MASK>

@@ -61,21 +61,33 @@ inline unsigned long long add_carry(unsigned h, unsigned l, unsigned below, unsi
 // The high word of hi:lo << n, for n in 1..31.
 __device__ __forceinline__ unsigned shl_high(unsigned hi, unsigned lo, unsigned n) { return (hi << n) | (lo >> (32u - n)); }
 
-// The largest of several operands' distances below 2^-511 as unsigned numbers: from kProductRange on, one of them
-// is outside 2^-511 .. 2^511 (or zero).
-constexpr unsigned kProductRange = 0x3FF00000u;
+// What the products below collect over any number of them: operands within
+// 2^-511 .. 2^511 are taken, whose product is normal; WIDE takes every normal
+// operand of a product well inside the normal range (two instructions more).
+template <bool WIDE>
+struct ProductRange {
+    unsigned operand = 0, result = 0;  // largest distance (as unsigned numbers) from the lowest exponent taken
+    __device__ __forceinline__ bool left() const {
+        return operand >= (WIDE ? 0x7FE00000u : 0x3FF00000u) || result >= 0x7FC00000u;
+    }
+};
 
-// a * b, rounded to nearest-even, for operands within 2^-511 .. 2^511 (whose
-// product is normal), without a branch: `range` collects what tells the caller,
-// after any number of products, that one was not (kProductRange), and that they
-// are to be done again in FP64.
-__device__ __forceinline__ double mul_rn_range(double a, double b, unsigned &range) {
+// a * b, rounded to nearest-even, without a branch; `range` tells the caller,
+// after any number of products, that an operand was not taken, and that they are
+// to be done again in FP64.
+template <bool WIDE>
+__device__ __forceinline__ double mul_rn_range(double a, double b, ProductRange<WIDE> &range) {
     const unsigned long long ia = (unsigned long long)__double_as_longlong(a);
     const unsigned long long ib = (unsigned long long)__double_as_longlong(b);
     const unsigned ahi = high_word(ia), alo = low_word(ia), bhi = high_word(ib), blo = low_word(ib);
     const unsigned ea = ahi & 0x7FF00000u, eb = bhi & 0x7FF00000u;  // the exponent fields, in place
-    const unsigned ra = ea - 0x20000000u, rb = eb - 0x20000000u, r2 = ra > rb ? ra : rb;
-    range = range > r2 ? range : r2;
+    const unsigned least = WIDE ? 0x00100000u : 0x20000000u;
+    const unsigned ra = ea - least, rb = eb - least, r2 = ra > rb ? ra : rb;
+    range.operand = range.operand > r2 ? range.operand : r2;
+    if (WIDE) {
+        const unsigned re = ea + eb - (1024u << 20);
+        range.result = range.result > re ? range.result : re;
+    }
     // significands, a's shifted left by 10: the product's high 64 bits h1:h0 lie in [2^50, 2^52), and the
     // middle word's sum stays below 2^64
     const unsigned ah = (shl_high(ahi, alo, 10) & 0x3FFFFFFFu) | 0x40000000u, al = alo << 10;
@@ -142,9 +154,9 @@ __device__ __forceinline__ double add_rn_int(double a, double b) {
 // add_rn_int for operands of nearby exponents, which need no other path.
 __device__ __forceinline__ double add_rn_near(double a, double b) { return add_rn_int(a, b); }
 __device__ __forceinline__ double mul_rn_int(double a, double b) {
-    unsigned range = 0;
+    ProductRange<false> range;
     const double r = mul_rn_range(a, b, range);
-    return range >= kProductRange ? mul_rn_hw(a, b) : r;
+    return range.left() ? mul_rn_hw(a, b) : r;
 }
 
 } // namespace f2c

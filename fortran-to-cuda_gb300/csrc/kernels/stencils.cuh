@@ -81,13 +81,13 @@ static __global__ void __launch_bounds__(kDiffBX *kDiffBY) diffusion7_kernel(con
     for (int k = k0; k < k1; ++k, q += plane) {
         const double west = __ldg(A + q - 1), east = __ldg(A + q + 1), south = __ldg(A + q - sx), north = __ldg(A + q + sx);
         const double above = __ldg(A + q + plane);
-        unsigned range = 0;
+        ProductRange<false> range;
         SumRange sums;
         const double first = add_rn_range(add_rn_range(west + east, south, sums), north, sums);
         const double num = (first + below + above) - mul_rn_range(6.0, centre, range);
         const double lap = folded ? num : divide(num, p.dx2);
         double r = centre + mul_rn_range(factor, lap, range);
-        if (range >= kProductRange || sums.left()) {
+        if (range.left() || sums.left()) {
             const double n = add_rn_hw(add_rn_hw(add_rn_hw(west, east), south), north) + below + above - mul_rn_hw(6.0, centre);
             r = centre + mul_rn_hw(p.dtnu, p.dx2_pow2 ? scale_pow2(n, -p.dx2_exp, 1.0 / p.dx2) : n / p.dx2);
         }
@@ -152,11 +152,11 @@ static __global__ void __launch_bounds__(kYeeBX *kYeeBY) yee_h_kernel(const YeeA
         if (j >= j1) return;
         const double north = __ldg(p.ez + q + p.sx), east = __ldg(p.ez + q + 1);
         const double hx = p.hx[q], hy = p.hy[q];
-        unsigned range = 0;
+        ProductRange<false> range;
         SumRange sums;
         double x = hx - mul_rn_range(p.ch, add_rn_range(north, sign_flipped(e), sums), range);
         double y = hy + mul_rn_range(p.ch, east - e, range);
-        if (range >= kProductRange || sums.left()) {
+        if (range.left() || sums.left()) {
             x = hx - mul_rn_hw(p.ch, north - e);
             y = hy + mul_rn_hw(p.ch, east - e);
         }
@@ -177,10 +177,10 @@ static __global__ void __launch_bounds__(kYeeBX *kYeeBY) yee_e_kernel(const YeeA
     for (int j = j0; j < j0 + kYeeJY; ++j, q += p.sx) {
         if (j >= j1) return;
         const double ez = p.ez[q], hy = __ldg(p.hy + q), west = __ldg(p.hy + q - 1), hx = __ldg(p.hx + q);
-        unsigned range = 0;
+        ProductRange<false> range;
         SumRange sums;
         double e = ez + mul_rn_range(p.ce, (hy - west) - add_rn_range(hx, sign_flipped(south), sums), range);
-        if (range >= kProductRange || sums.left()) e = ez + mul_rn_hw(p.ce, (hy - west) - (hx - south));
+        if (range.left() || sums.left()) e = ez + mul_rn_hw(p.ce, (hy - west) - (hx - south));
         p.ez[q] = e;
         south = hx;
     }

@@ -25,7 +25,7 @@ static inline int __clzll(long long x) { return x == 0 ? 64 : __builtin_clzll((u
 int main(int argc, char **argv) {
     const uint64_t n = argc > 1 ? std::strtoull(argv[1], nullptr, 10) : 1000000;
     int failed = 0;
-    for (int op = 0; op < 2; ++op)
+    for (int op = 0; op < 3; ++op)
         for (int dist = 0; dist < 7; ++dist)
             for (uint64_t i = 0; i < n; ++i) {
                 uint64_t ia, ib;
@@ -35,11 +35,16 @@ int main(int argc, char **argv) {
                 const double want = op ? __dmul_rn(a, b) : __dadd_rn(a, b);
                 double got;
                 bool left, may;
-                if (op) {
-                    unsigned range = 0;
+                if (op == 1) {
+                    f2c::ProductRange<false> range;
                     got = f2c::mul_rn_range(a, b, range);
-                    left = range >= f2c::kProductRange;
+                    left = range.left();
                     may = ea < 512 || ea > 1534 || eb < 512 || eb > 1534;
+                } else if (op == 2) {
+                    f2c::ProductRange<true> range;
+                    got = f2c::mul_rn_range(a, b, range);
+                    left = range.left();
+                    may = ea == 0 || eb == 0 || ea == 0x7FF || eb == 0x7FF || ea + eb < 1024 || ea + eb >= 1024 + 2044;
                 } else {
                     f2c::SumRange range;
                     got = f2c::add_rn_range(a, b, range);
