@@ -151,9 +151,9 @@ static __device__ __noinline__ void fast_point_fp64(const AdvArgs &a, int i, int
 
 // An 8-byte copy from global to shared memory that runs on while the thread does (cp.async).
 __device__ __forceinline__ void fetch(long long *to, const double *from) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
 }
-__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;"); }
+__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
@@ -322,9 +322,9 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
                 const int g = f < 3 ? f : 3;
                 double *o = f < 3 ? a.out[f] : a.st[f - 3];
                 bool fits;
-                double t = wide_result(T, e, c.wide_hi[g], c.wide_lo[g], c.wide_e[g], fits);
+                const double t = wide_result<ADVANCE>(T, e, c.wide_hi[g], c.wide_lo[g], c.wide_e[g],
+                                                      ADVANCE ? old[ADVANCE ? f : 0] : 0.0, fits);
                 if (!fits || e - used > kWideSlack) slow |= 1u << f;
-                if (ADVANCE) t += old[ADVANCE ? f : 0];
                 if (!o) return;
                 if (images) store_filled(o, f == 2 ? 1 : 0, a, i, j, k, t);
                 else o[p] = t;

@@ -127,21 +127,28 @@ __device__ __forceinline__ void wide_scale(Wide &w, long long r) {
     w.m = s.value() << 2;
 }
 
-// T * 2^e * k, for the coefficient k whose words are `khi`, `klo` with the sum's
-// constant 2^-offset taken off the exponent field; `ke` is that field less one.
-// The conversion rounds T to 53 bits, the product rounds once more. Where the
-// factor is below the normal range the product is taken 2^512 larger first (the
-// results there are subnormal or zero); above it `fits` is cleared.
-__device__ __forceinline__ double wide_result(long long T, int e, int khi, int klo, int ke, bool &fits) {
+// T * 2^e * k (plus `old` where ADD), for the coefficient k whose words are
+// `khi`, `klo` with the sum's constant 2^-offset taken off the exponent field;
+// `ke` is that field less one. The conversion rounds T to 53 bits, the product
+// (or multiply-add) rounds once more. Where the factor is below the normal range
+// the product is taken 2^512 larger first (the results there are subnormal or
+// zero); above it `fits` is cleared.
+template <bool ADD>
+__device__ __forceinline__ double wide_result(long long T, int e, int khi, int klo, int ke, double old, bool &fits) {
     double t;
     asm("cvt.rn.f64.s64 %0, %1;" : "=d"(t) : "l"(T));
     fits = true;
+    double factor = __hiloint2double(khi + (e << 20), klo);
     if ((unsigned)(e + ke) >= 2046u) {
         if (e + ke >= 2046) fits = T == 0;
-        if (e + ke < -500 || T == 0) return 0.0;
-        return t * __hiloint2double(khi + ((e + 512) << 20), klo) * 0x1p-512;
+        if (e + ke < -500 || T == 0) {
+            factor = 0.0;
+        } else {
+            t *= __hiloint2double(khi + ((e + 512) << 20), klo);
+            factor = 0x1p-512;
+        }
     }
-    return t * __hiloint2double(khi + (e << 20), klo);
+    return ADD ? __fma_rn(t, factor, old) : t * factor;
 }
 
 } // namespace f2c
