@@ -282,12 +282,15 @@ def load() -> ctypes.CDLL:
                        ("poll", [u64, ctypes.POINTER(ServeDone), ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)]),
                        ("drain", [u64, ctypes.c_double]),
                        ("result", [u64, u64, ctypes.c_int32, ctypes.POINTER(ctypes.POINTER(ctypes.c_double))]),
+                       ("take", [u64, u64, ctypes.c_int32, ctypes.POINTER(ctypes.c_void_p)]),
                        ("release", [u64, u64]),
                        ("stats_get", [u64, ctypes.POINTER(ServeStats)]),
                        ("destroy", [u64])):
         fn = getattr(lib, f"f2c_serve_{name}_v1")
         fn.argtypes = args
         fn.restype = ctypes.c_int
+    lib.f2c_serve_free_v1.argtypes = [ctypes.c_void_p]
+    lib.f2c_serve_free_v1.restype = None
     lib.f2c_serve_clock_v1.argtypes = [u64]
     lib.f2c_serve_clock_v1.restype = ctypes.c_double
     lib.f2c_serve_error_v1.argtypes = [u64]

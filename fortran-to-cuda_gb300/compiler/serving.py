@@ -100,6 +100,22 @@ class ServeError(RuntimeError):
     pass
 
 
+class _Taken:
+    """A field taken from the native server, as the memory behind a numpy array: freed with the last view of it.
+
+    Taking the field replaces a copy into new memory, whose page faults made it 40 of the 76 ms of a run that keeps
+    the results of twelve jobs (542 MB).
+    """
+
+    def __init__(self, lib, address: int, shape):
+        self._lib = lib
+        self._address = address
+        self.__array_interface__ = {"data": (address, False), "shape": tuple(shape), "typestr": "<f8", "version": 3}
+
+    def __del__(self):
+        self._lib.f2c_serve_free_v1(self._address)
+
+
 class Server:
     """Continuous batching through the native server, on a residency domain of its own.
 
@@ -181,9 +197,9 @@ class Server:
                 shape = job.geometry.shape
                 out = []
                 for f in range(3 + job.nscalar):
-                    ptr = ctypes.POINTER(ctypes.c_double)()
-                    self._check(lib.f2c_serve_result_v1(server, r.id, f, ctypes.byref(ptr)), server)
-                    out.append(np.ctypeslib.as_array(ptr, shape=shape).copy())
+                    ptr = ctypes.c_void_p()
+                    self._check(lib.f2c_serve_take_v1(server, r.id, f, ctypes.byref(ptr)), server)
+                    out.append(np.asarray(_Taken(lib, ptr.value, shape)))
                 job.result = out
                 self._check(lib.f2c_serve_release_v1(server, r.id), server)
         stats = native.ServeStats()

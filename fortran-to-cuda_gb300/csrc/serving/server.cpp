@@ -853,9 +853,28 @@ extern "C" int f2c_serve_result_v1(f2c_server_t server, uint64_t id, int32_t fie
     if (it == s->results.end()) return fail(FORT_SCOPE_STALE, "no kept result for this job");
     Job *j = it->second.get();
     if (field < 0 || field >= j->fields) return fail(FORT_SCOPE_ARGUMENT, "field index out of range");
+    if (!j->host[j->result_set][field]) return fail(FORT_SCOPE_STALE, "the field has been taken");
     *host = static_cast<const double *>(j->host[j->result_set][field]);
     return FORT_SCOPE_OK;
 }
+
+extern "C" int f2c_serve_take_v1(f2c_server_t server, uint64_t id, int32_t field, double **host) {
+    Server *s = find(server);
+    if (!s) return fail(FORT_SCOPE_STALE, "unknown server");
+    if (!host) return fail(FORT_SCOPE_ARGUMENT, "null result output");
+    std::lock_guard<std::mutex> g(s->lock);
+    auto it = s->results.find(id);
+    if (it == s->results.end()) return fail(FORT_SCOPE_STALE, "no kept result for this job");
+    Job *j = it->second.get();
+    if (field < 0 || field >= j->fields) return fail(FORT_SCOPE_ARGUMENT, "field index out of range");
+    void *&mine = j->host[j->result_set][field];
+    if (!mine) return fail(FORT_SCOPE_STALE, "the field has been taken");
+    *host = static_cast<double *>(mine);
+    mine = nullptr;
+    return FORT_SCOPE_OK;
+}
+
+extern "C" void f2c_serve_free_v1(double *host) { std::free(host); }
 
 extern "C" int f2c_serve_release_v1(f2c_server_t server, uint64_t id) {
     Server *s = find(server);

@@ -121,6 +121,11 @@ int f2c_serve_drain_v1(f2c_server_t server, double timeout_s);
  * 3.. scalars), padded layout, valid until f2c_serve_release_v1. */
 int f2c_serve_result_v1(f2c_server_t server, uint64_t id, int32_t field, const double **host);
 int f2c_serve_release_v1(f2c_server_t server, uint64_t id);
+/* The same array, handed over instead of lent: it outlives the result's release
+ * and the server, and the caller frees it with f2c_serve_free_v1. A field is
+ * taken once; f2c_serve_result_v1 refuses it afterwards (FORT_SCOPE_STALE). */
+int f2c_serve_take_v1(f2c_server_t server, uint64_t id, int32_t field, double **host);
+void f2c_serve_free_v1(double *host);
 int f2c_serve_stats_get_v1(f2c_server_t server, f2c_serve_stats_v1 *stats);
 /* Last failure text of the server (never NULL). */
 const char *f2c_serve_error_v1(f2c_server_t server);
