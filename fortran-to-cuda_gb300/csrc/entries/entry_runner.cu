@@ -594,6 +594,7 @@ int run(const EntryCall &call) {
         diff.a = dev(1);
         diff.dtnu = *call.reals[0] * *call.reals[1];
         diff.dx2 = *call.reals[2] * *call.reals[2];
+        diff.dx2_positive = diff.dx2 > 0.0;
         diff.dx2_pow2 = power_of_two(diff.dx2, &diff.dx2_exp) ? 1 : 0;
         diff.nx = (int)g.n[0]; diff.ny = (int)g.n[1]; diff.nz = (int)g.n[2]; diff.h = (int)g.h;
         diff.sx = sx; diff.plane = plane;
@@ -604,7 +605,7 @@ int run(const EntryCall &call) {
         argument = &diff;
         argument_size = sizeof diff;
     } else if (t == Template::Jacobi) {
-        jac = JacobiArgs{dev(1), dev(0), (int)g.n[0], (int)g.n[1], (int)g.h, sx};
+        jac = JacobiArgs{dev(1), dev(0), (int)g.n[0], (int)g.n[1], (int)g.h, sx, 0};
         kernel.function = (const void *)jacobi5_kernel;
         const dim3 grid = jacobi_grid(jac);
         kernel.grid[0] = grid.x; kernel.grid[1] = grid.y; kernel.grid[2] = grid.z;

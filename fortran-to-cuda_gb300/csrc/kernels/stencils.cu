@@ -24,11 +24,13 @@ extern "C" int f2c_diffusion7_v1(const f2c_grid_v1 *grid, const double *a, doubl
     p.b = b;
     p.dtnu = dt * nu;
     p.dx2 = grid->dx * grid->dx;
+    p.dx2_positive = p.dx2 > 0.0;
     p.dx2_pow2 = power_of_two(p.dx2, &p.dx2_exp) ? 1 : 0;
     p.nx = (int)grid->nx; p.ny = (int)grid->ny; p.nz = (int)grid->nz; p.h = (int)grid->halo;
     p.sx = grid->sx;
     p.plane = grid->sx * grid->sy;
-    diffusion7_kernel<<<diffusion_grid(p), dim3(kDiffBX, kDiffBY, 1), 0, static_cast<cudaStream_t>(stream)>>>(p);
+    const dim3 blocks = diffusion_grid(p);
+    diffusion7_kernel<<<blocks, dim3(kDiffBX, kDiffBY, 1), 0, static_cast<cudaStream_t>(stream)>>>(p);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : fail(6, std::string("diffusion launch: ") + cudaGetErrorString(e));
 }
@@ -44,8 +46,9 @@ extern "C" int f2c_jacobi5_v1(const double *u, double *v, int64_t nx, int64_t ny
     if (int s = check_plane(nx, ny, halo, sx)) return s;
     if (!u || !v) return fail(1, "null Jacobi field");
     if (u == v) return fail(3, "Jacobi output aliases its input");
-    JacobiArgs p{u, v, (int)nx, (int)ny, (int)halo, sx};
-    jacobi5_kernel<<<jacobi_grid(p), dim3(kJacBX, kJacBY, 1), 0, static_cast<cudaStream_t>(stream)>>>(p);
+    JacobiArgs p{u, v, (int)nx, (int)ny, (int)halo, sx, 0};
+    const dim3 blocks = jacobi_grid(p);
+    jacobi5_kernel<<<blocks, dim3(kJacBX, kJacBY, 1), 0, static_cast<cudaStream_t>(stream)>>>(p);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : fail(6, std::string("Jacobi launch: ") + cudaGetErrorString(e));
 }

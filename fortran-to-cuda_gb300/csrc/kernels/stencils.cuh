@@ -13,6 +13,7 @@
 
 #include <cstdint>
 
+#include "device.cuh"
 #include "soft_fp64.cuh"
 
 // FP64 additions bound these stencils (1.68 lanes a clock per SM), so the
@@ -21,6 +22,11 @@
 // branches: a point whose operands they cannot take is done again in FP64. The
 // additions moved are ones along y: a zero of the west or east boundary would
 // send a warp of every row that way, one of the others only the outer rows'.
+// A diffusion warp that sees a zero among the values its integer operations
+// would read (a region at rest, an outer row) goes to FP64 at once instead of
+// doing the point twice: 256^3 of zeros 0.48 -> 0.33 ms with dx 1, 1.63 -> 0.33
+// with dx 0.3. In the Yee kernels the same choice cost fields without zeros more
+// (0.238 -> 0.249 ms at 4096^2) than it gave those of zeros (107 -> 99 us at 2048^2).
 namespace f2c {
 
 // x * 2^e for an exact power-of-two factor, on the integer pipe when the
@@ -46,31 +52,55 @@ __device__ __forceinline__ double sign_flipped(double x) {
     return __longlong_as_double((long long)r);
 }
 
+// A value whose high word is zero but for the sign: zero, or far below what the integer operations take.
+__device__ __forceinline__ bool nearly_zero(unsigned a, unsigned b, unsigned c) { return min(min(a << 1, b << 1), c << 1) == 0; }
+
 // The division where dx*dx is no power of two, out of line (inline it is evaluated for every point).
 static __device__ __noinline__ double divide(double x, double y) { return x / y; }
+// The same where y > 0 (dx*dx and not NaN), without a zero numerator's slow path: 0 / y is that zero.
+__device__ __forceinline__ double quotient(double x, double y, bool positive) {
+    if (positive && ((unsigned long long)__double_as_longlong(x) << 1) == 0) return x;
+    return divide(x, y);
+}
 
 struct DiffusionArgs {
     const double *a;
     double *b;
     double dtnu;      // dt*nu, formed on the host exactly as the source does
     double dx2;       // dx*dx
+    int dx2_positive; // dx*dx > 0 (a NaN is not)
     int dx2_pow2;     // dx*dx is 2^dx2_exp: the division is an exact scaling
     int dx2_exp;
     int nx, ny, nz, h;
     long long sx, plane;
+    int kz;           // levels per z-chunk (diffusion_grid)
 };
 
 constexpr int kDiffBX = 32, kDiffBY = 8, kDiffKZ = 32;
 
-// 384^3: 0.59 ms with two of the seven additions on the integer pipes (0.79 with
+// The point in FP64 (one call, so that the common path issues none of it).
+static __device__ __noinline__ double diffusion_fp64(const DiffusionArgs &p, double west, double east, double south, double north,
+                                                     double below, double above, double centre) {
+    const double n = west + east + south + north + below + above - 6.0 * centre;
+    const long long b = __double_as_longlong(n);
+    const int ex = (int)((unsigned long long)b >> 52) & 0x7ff, r = ex - p.dx2_exp;
+    double lap;
+    if (p.dx2_pow2 && ex != 0 && ex != 0x7ff && r >= 1 && r <= 0x7fe) lap = __longlong_as_double(b - ((long long)p.dx2_exp << 52));
+    else lap = quotient(n, p.dx2, p.dx2_positive);
+    return centre + p.dtnu * lap;
+}
+
+// 384^3: 0.575 ms (0.59 before the chunk depths and the choice above) with two of the seven additions on the integer pipes (0.79 with
 // none, 0.70 with one, 0.69 with three: an addition there takes 50 ALU
 // instructions, an FP64 one the time of 38).
-static __global__ void __launch_bounds__(kDiffBX *kDiffBY) diffusion7_kernel(const DiffusionArgs p) {
+static __global__ void __launch_bounds__(kDiffBX *kDiffBY) diffusion7_kernel(const __grid_constant__ DiffusionArgs p) {
     const int i = blockIdx.x * kDiffBX + threadIdx.x;
     const int j = blockIdx.y * kDiffBY + threadIdx.y;
-    if (i >= p.nx || j >= p.ny) return;
-    const int k0 = blockIdx.z * kDiffKZ;
-    const int k1 = min(k0 + kDiffKZ, p.nz);
+    const bool active = i < p.nx && j < p.ny;
+    const unsigned lanes = __ballot_sync(0xffffffffu, active);
+    if (!active) return;
+    const int k0 = blockIdx.z * p.kz;
+    const int k1 = min(k0 + p.kz, p.nz);
     const double *__restrict__ A = p.a;
     const long long sx = p.sx, plane = p.plane;
     long long q = (long long)(i + p.h) + sx * (long long)(j + p.h) + plane * (long long)(k0 + p.h);
@@ -81,16 +111,19 @@ static __global__ void __launch_bounds__(kDiffBX *kDiffBY) diffusion7_kernel(con
     for (int k = k0; k < k1; ++k, q += plane) {
         const double west = __ldg(A + q - 1), east = __ldg(A + q + 1), south = __ldg(A + q - sx), north = __ldg(A + q + sx);
         const double above = __ldg(A + q + plane);
-        ProductRange<false> range;
-        SumRange sums;
-        const double first = add_rn_range(add_rn_range(west + east, south, sums), north, sums);
-        const double num = (first + below + above) - mul_rn_range(6.0, centre, range);
-        const double lap = folded ? num : divide(num, p.dx2);
-        double r = centre + mul_rn_range(factor, lap, range);
-        if (range.left() || sums.left()) {
-            const double n = add_rn_hw(add_rn_hw(add_rn_hw(west, east), south), north) + below + above - mul_rn_hw(6.0, centre);
-            r = centre + mul_rn_hw(p.dtnu, p.dx2_pow2 ? scale_pow2(n, -p.dx2_exp, 1.0 / p.dx2) : n / p.dx2);
+        bool again = __any_sync(lanes, nearly_zero((unsigned)__double2hiint(centre), (unsigned)__double2hiint(south),
+                                                   (unsigned)__double2hiint(north)));
+        double r;
+        if (!again) {
+            ProductRange<false> range;
+            SumRange sums;
+            const double first = add_rn_range(add_rn_range(west + east, south, sums), north, sums);
+            const double num = (first + below + above) - mul_rn_range(6.0, centre, range);
+            const double lap = folded ? num : divide(num, p.dx2);
+            r = centre + mul_rn_range(factor, lap, range);
+            again = range.left() || sums.left();
         }
+        if (again) r = diffusion_fp64(p, west, east, south, north, below, above, centre);
         p.b[q] = r;
         below = centre;
         centre = above;
@@ -102,20 +135,21 @@ struct JacobiArgs {
     double *v;
     int nx, ny, h;
     long long sx;
+    int rows;  // rows a thread does (jacobi_grid)
 };
 
-constexpr int kJacBX = 64, kJacBY = 4, kJacJY = 8;  // each thread does kJacJY rows
+constexpr int kJacBX = 64, kJacBY = 4, kJacJY = 8;  // most rows a thread does
 
 // 8192^2: 0.27 ms with one of the three additions on the integer pipes (0.39 with
 // none, 0.34 with three in two rows).
 static __global__ void __launch_bounds__(kJacBX *kJacBY) jacobi5_kernel(const JacobiArgs p) {
     const int i = blockIdx.x * kJacBX + threadIdx.x;
-    const int j0 = (blockIdx.y * kJacBY + threadIdx.y) * kJacJY;
+    const int j0 = (blockIdx.y * kJacBY + threadIdx.y) * p.rows;
     if (i >= p.nx) return;
     const double *__restrict__ U = p.u;
     const long long sx = p.sx;
     long long q = (long long)(i + p.h) + sx * (long long)(j0 + p.h);
-    const int j1 = min(j0 + kJacJY, p.ny);
+    const int j1 = min(j0 + p.rows, p.ny);
     double south = j0 < p.ny ? __ldg(U + q - sx) : 0.0;
     double centre = j0 < p.ny ? __ldg(U + q) : 0.0;
     for (int j = j0; j < j1; ++j, q += sx) {
@@ -186,11 +220,34 @@ static __global__ void __launch_bounds__(kYeeBX *kYeeBY) yee_e_kernel(const YeeA
     }
 }
 
-inline dim3 diffusion_grid(const DiffusionArgs &p) {
-    return dim3((p.nx + kDiffBX - 1) / kDiffBX, (p.ny + kDiffBY - 1) / kDiffBY, (p.nz + kDiffKZ - 1) / kDiffKZ);
+// Levels of a z-chunk: the depth with the least time on the SM with the most
+// CTAs, as the strict advection kernel's (chunk_depth); a deep march on a small
+// grid is one long serial chain. 26 x 26 x 156: 7.8 us a step (23 at 32 levels, with
+// every addition in FP64).
+inline dim3 diffusion_grid(DiffusionArgs &p) {
+    const unsigned gx = (p.nx + kDiffBX - 1) / kDiffBX, gy = (p.ny + kDiffBY - 1) / kDiffBY;
+    const long long sms = current_sm_count();
+    long long best = -1;
+    for (int kz = 1; kz <= kDiffKZ && kz <= p.nz; ++kz) {
+        const long long ctas = (long long)gx * gy * ((p.nz + kz - 1) / kz);
+        const long long cost = ((ctas + sms - 1) / sms + 1) * (2 * kz + 1);
+        if (best < 0 || cost <= best) {
+            best = cost;
+            p.kz = kz;
+        }
+    }
+    return dim3(gx, gy, (p.nz + p.kz - 1) / p.kz);
 }
-inline dim3 jacobi_grid(const JacobiArgs &p) {
-    return dim3((p.nx + kJacBX - 1) / kJacBX, (p.ny + kJacBY * kJacJY - 1) / (kJacBY * kJacJY), 1);
+// Rows of a thread: as many (8, 4, 2 or 1) as leave kJacCtas CTAs per SM; the
+// rows of a thread are one serial chain. 251 x 5541: 10.4 us a sweep (13.1 at 8 rows,
+// with every addition in FP64).
+constexpr int kJacCtas = 8;
+inline dim3 jacobi_grid(JacobiArgs &p) {
+    const unsigned gx = (p.nx + kJacBX - 1) / kJacBX;
+    const long long wanted = (long long)kJacCtas * current_sm_count();
+    p.rows = kJacJY;
+    while (p.rows > 1 && (long long)gx * ((p.ny + kJacBY * p.rows - 1) / (kJacBY * p.rows)) < wanted) p.rows /= 2;
+    return dim3(gx, (p.ny + kJacBY * p.rows - 1) / (kJacBY * p.rows), 1);
 }
 inline dim3 yee_grid(const YeeArgs &p) { return dim3((p.nx + kYeeBX - 1) / kYeeBX, (p.ny + kYeeBY * kYeeJY - 1) / (kYeeBY * kYeeJY), 1); }
 
