@@ -24,7 +24,10 @@
 // forms' differences are computed on the integer pipes (soft_fp64.cuh, rounded
 // exactly as DMUL and DADD), without branches: the operands that those do not
 // take (zeros at the walls among them) have the thread do its half of the level
-// again in FP64. Operation count per point: U, V, W: 9 face sums + 18 flux
+// again in FP64. A warp that starts a chunk beside zero velocities (a region at
+// rest, a flow without W) takes the products they are in in FP64 from the start:
+// 256 x 256 x 128 with W zero 1.77 -> 1.29 ms, at rest 1.77 -> 1.60 (a choice
+// level by level cost fields without zeros 4 %). Operation count per point: U, V, W: 9 face sums + 18 flux
 // products + 15 flux differences + 48 advective-form operations = 90; scalars: 3
 // shared coefficient products + 11 per scalar. Of the 126 with three scalars 69
 // are left to the FP64 pipe. Measured at 512 x 512 x 128 without and with three
@@ -33,11 +36,13 @@
 // differences as well; 4.37 and 6.99 with the nine face sums instead, 4.72 and
 // 6.77 with the differences and the advecting sums (registers: 72 a thread). On
 // the sine-mode fields with a Gaussian tracer: 3.95 and 6.02 ms (7.13 before;
-// 7.01 with one range for momentum and scalars, whose tails then cost both).
+// 7.01 with one range for momentum and scalars, whose tails then cost both; 5.93
+// with the warps beside zeros apart).
 #pragma once
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "advection_kernels.cuh"
 #include "device.cuh"
@@ -83,6 +88,12 @@ __device__ __forceinline__ double opaque_negate(double x) {
     asm("xor.b64 %0, %1, 0x8000000000000000;" : "=l"(r) : "l"((unsigned long long)__double_as_longlong(x)));
     return __longlong_as_double((long long)r);
 }
+
+// Whether the high word is zero but for the sign (zero, or far below what the integer products take).
+__device__ __forceinline__ bool zero_high(double x) { return ((unsigned)__double2hiint(x) << 1) == 0; }
+
+// What a warp does in FP64 at once (faces_tile).
+constexpr int kRestW = 1, kRest = 2;
 
 // A read-only global load the compiler must issue where it stands (not merged
 // with an earlier load of the same address), so that a value loaded before the
@@ -137,11 +148,14 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
 
     // Top-face fluxes of the level below the current one (bottom faces), carried up the march.
     double FUzb = 0.0, FVzb = 0.0, FWzb = 0.0, ftb[NS > 0 ? NS : 1];
+    bool still = false, still_w = false;  // U or V, and W, are zero here
     if (active) {
         // prologue: top faces of level k0-1
         const double Um = LD(U, p, 0, 0, -1), U0 = LD(U, p, 0, 0, 0);
         const double Vm = LD(V, p, 0, 0, -1), V0 = LD(V, p, 0, 0, 0);
         const double Wm = LD(W, p, 0, 0, -1), W0 = LD(W, p, 0, 0, 0);
+        still = zero_high(U0) || zero_high(V0);
+        still_w = zero_high(W0) && zero_high(Wm);
         if (DO_U) {
             const double sUz = U0 + Um;
             const double sWx = LD(W, p, 1, 0, -1) + Wm;
@@ -163,8 +177,12 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
         }
     }
 
+    // A warp that starts beside zero velocities takes the products they are in (kRestW: W's, kRest: all) in FP64 at
+    // once. Its choice for the chunk.
+    const int rest = (__any_sync(0xffffffffu, still) ? kRest : 0) | (__any_sync(0xffffffffu, still_w) ? kRestW : 0);
     int buf = 0;
-    for (int k = k0; k < k1; ++k, p += plane, pw += plane, buf ^= 1) {
+    auto level = [&](const int k, auto resting) {
+        constexpr bool REST = decltype(resting)::value;
         double *xf = xface + buf * NF * Smem::XF;
         double *yf = yface + buf * NF * Smem::YF;
         // ---------------- phase A: own east / north / top faces, edge faces ----------------
@@ -194,26 +212,35 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
             if (DO_U || DO_W) sUz = Up + U0;
             if (DO_V || DO_W) sVz = Vp + V0;
             if (DO_W) sWz = Wp + W0;
-            auto fluxes = [&](auto mul) {
+            // which: 1 the fluxes without W, 2 those with it, 3 all
+            auto fluxes = [&](auto which, auto mul) {
+                constexpr bool UV = decltype(which)::value & 1, WITH_W = decltype(which)::value & 2;
                 if (DO_U) {
-                    FUx = mul(mul(c.Ax, sUx), sUx);
-                    FUy = mul(mul(c.Ay, sUy), sVx);
-                    FUz = mul(mul(c.Az, sUz), sWx);
+                    if (UV) FUx = mul(mul(c.Ax, sUx), sUx);
+                    if (UV) FUy = mul(mul(c.Ay, sUy), sVx);
+                    if (WITH_W) FUz = mul(mul(c.Az, sUz), sWx);
                 }
                 if (DO_V) {
-                    FVx = mul(mul(c.Ax, sVx), sUy);
-                    FVy = mul(mul(c.Ay, sVy), sVy);
-                    FVz = mul(mul(c.Az, sVz), sWy);
+                    if (UV) FVx = mul(mul(c.Ax, sVx), sUy);
+                    if (UV) FVy = mul(mul(c.Ay, sVy), sVy);
+                    if (WITH_W) FVz = mul(mul(c.Az, sVz), sWy);
                 }
-                if (DO_W) {
+                if (DO_W && WITH_W) {
                     FWx = mul(mul(c.Ax, sWx), sUz);
                     FWy = mul(mul(c.Ay, sWy), sVz);
                     FWz = mul(mul(c.Az, sWz), sWz);
                 }
             };
-            ProductRange<false> range;
-            fluxes([&](double x, double y) { return mul_rn_range(x, y, range); });
-            if (range.left()) fluxes([](double x, double y) { return mul_rn_hw(x, y); });
+            auto fp64 = [](double x, double y) { return x * y; };
+            if (REST) fluxes(std::integral_constant<int, 2>{}, fp64);
+            if (REST && (rest & kRest)) {
+                fluxes(std::integral_constant<int, 1>{}, fp64);
+            } else {
+                constexpr std::integral_constant<int, REST ? 1 : 3> which{};
+                ProductRange<false> range;
+                fluxes(which, [&](double x, double y) { return mul_rn_range(x, y, range); });
+                if (range.left()) fluxes(which, [](double x, double y) { return mul_rn_hw(x, y); });
+            }
             if (NS > 0) {
                 // a scalar's own range: a tracer's zeros and tails (which WIDE takes further down) cost its own products only
                 ProductRange<true> shared;
@@ -319,29 +346,38 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
             const double Vw = LD(V, p, -1, 0, 0), Vs = LD(V, p, 0, -1, 0), Vm = LD(V, p, 0, 0, -1);
             const double Ww = LD(W, p, -1, 0, 0), Ws = LD(W, p, 0, -1, 0), Wm = LD(W, p, 0, 0, -1);
             double aU[3] = {0, 0, 0}, aV[3] = {0, 0, 0}, aW[3] = {0, 0, 0};  // the advective forms' terms
-            auto advective = [&](auto mul, auto sub) {
+            auto advective = [&](auto which, auto mul, auto sub) {
+                constexpr bool UV = decltype(which)::value & 1, WITH_W = decltype(which)::value & 2;
                 if (DO_U) {
-                    aU[0] = mul(mul(c.Bux, sub(LDA(U, 1, 0, 0), Uw)), Uc);
-                    aU[1] = mul(mul(c.Buy, sub(LDA(U, 0, 1, 0), Us)), (sVx + Vs) + LD(V, p, 1, -1, 0));
-                    aU[2] = mul(mul(c.Buz, sub(LDA(U, 0, 0, 1), Um)), (sWx + Wm) + LD(W, p, 1, 0, -1));
+                    if (UV) aU[0] = mul(mul(c.Bux, sub(LDA(U, 1, 0, 0), Uw)), Uc);
+                    if (UV) aU[1] = mul(mul(c.Buy, sub(LDA(U, 0, 1, 0), Us)), (sVx + Vs) + LD(V, p, 1, -1, 0));
+                    if (WITH_W) aU[2] = mul(mul(c.Buz, sub(LDA(U, 0, 0, 1), Um)), (sWx + Wm) + LD(W, p, 1, 0, -1));
                 }
                 if (DO_V) {
-                    aV[0] = mul(mul(c.Bvx, sub(LDA(V, 1, 0, 0), Vw)), (sUy + Uw) + LD(U, p, -1, 1, 0));
-                    aV[1] = mul(mul(c.Bvy, sub(LDA(V, 0, 1, 0), Vs)), Vc);
-                    aV[2] = mul(mul(c.Bvz, sub(LDA(V, 0, 0, 1), Vm)), (sWy + Wm) + LD(W, p, 0, 1, -1));
+                    if (UV) aV[0] = mul(mul(c.Bvx, sub(LDA(V, 1, 0, 0), Vw)), (sUy + Uw) + LD(U, p, -1, 1, 0));
+                    if (UV) aV[1] = mul(mul(c.Bvy, sub(LDA(V, 0, 1, 0), Vs)), Vc);
+                    if (WITH_W) aV[2] = mul(mul(c.Bvz, sub(LDA(V, 0, 0, 1), Vm)), (sWy + Wm) + LD(W, p, 0, 1, -1));
                 }
-                if (DO_W) {
+                if (DO_W && WITH_W) {
                     aW[0] = mul(mul(c.Bwx, sub(LDA(W, 1, 0, 0), Ww)), (sUz + Uw) + LD(U, p, -1, 0, 1));
                     aW[1] = mul(mul(c.Bwy, sub(LDA(W, 0, 1, 0), Ws)), (sVz + Vs) + LD(V, p, 0, -1, 1));
                     aW[2] = mul(mul(c.Bwz, sub(LDA(W, 0, 0, 1), Wm)), Wc);
                 }
             };
-            ProductRange<false> range;
-            SumRange sums;
-            advective([&](double x, double y) { return mul_rn_range(x, y, range); },
-                      [&](double x, double y) { return add_rn_range(x, opaque_negate(y), sums); });
-            if (range.left() || sums.left())
-                advective([](double x, double y) { return mul_rn_hw(x, y); }, [](double x, double y) { return x - y; });
+            auto fp64 = [](double x, double y) { return x * y; };
+            auto difference = [](double x, double y) { return x - y; };
+            if (REST) advective(std::integral_constant<int, 2>{}, fp64, difference);
+            if (REST && (rest & kRest)) {
+                advective(std::integral_constant<int, 1>{}, fp64, difference);
+            } else {
+                constexpr std::integral_constant<int, REST ? 1 : 3> which{};
+                ProductRange<false> range;
+                SumRange sums;
+                advective(which, [&](double x, double y) { return mul_rn_range(x, y, range); },
+                          [&](double x, double y) { return add_rn_range(x, opaque_negate(y), sums); });
+                if (range.left() || sums.left())
+                    advective(which, [](double x, double y) { return mul_rn_hw(x, y); }, difference);
+            }
             if (DO_U) {
                 const double r = opaque_negate(((xf[0 * Smem::XF + xo] - xf[0 * Smem::XF + xw]) + (yf[0 * Smem::YF + yo] - yf[0 * Smem::YF + ys])) + (FUz - FUzb));
                 if (a.out[0]) store_point_t<FILL>(a.out[0], U, p, exact_half(r - ((aU[0] + aU[1]) + aU[2])), a, 0, i, j, k);
@@ -366,6 +402,11 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
             }
 #undef LDA
         }
+    };
+    if (rest) {
+        for (int k = k0; k < k1; ++k, p += plane, pw += plane, buf ^= 1) level(k, std::true_type{});
+    } else {
+        for (int k = k0; k < k1; ++k, p += plane, pw += plane, buf ^= 1) level(k, std::false_type{});
     }
 #undef LD
 }
