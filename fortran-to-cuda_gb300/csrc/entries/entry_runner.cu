@@ -595,6 +595,7 @@ int run(const EntryCall &call) {
         diff.dtnu = *call.reals[0] * *call.reals[1];
         diff.dx2 = *call.reals[2] * *call.reals[2];
         diff.dx2_positive = diff.dx2 > 0.0;
+        reciprocal_of(diff.dx2, &diff.high, &diff.low);
         diff.dx2_pow2 = power_of_two(diff.dx2, &diff.dx2_exp) ? 1 : 0;
         diff.nx = (int)g.n[0]; diff.ny = (int)g.n[1]; diff.nz = (int)g.n[2]; diff.h = (int)g.h;
         diff.sx = sx; diff.plane = plane;

@@ -25,6 +25,7 @@ extern "C" int f2c_diffusion7_v1(const f2c_grid_v1 *grid, const double *a, doubl
     p.dtnu = dt * nu;
     p.dx2 = grid->dx * grid->dx;
     p.dx2_positive = p.dx2 > 0.0;
+    reciprocal_of(p.dx2, &p.high, &p.low);
     p.dx2_pow2 = power_of_two(p.dx2, &p.dx2_exp) ? 1 : 0;
     p.nx = (int)grid->nx; p.ny = (int)grid->ny; p.nz = (int)grid->nz; p.h = (int)grid->halo;
     p.sx = grid->sx;

@@ -69,6 +69,23 @@ def test_diffusion(cuda, how, dx, n):
     assert np.array_equal(_bits(out.cpu().numpy()), _bits(ref))
 
 
+@pytest.mark.parametrize("dx", [0.1, 0.7, 1.0 / 3.0, 1.0 + 2.0**-52, 2.0 - 2.0**-52, 1e-20, 3e45, 1e-90, 1.5 * 2.0**-128])
+def test_diffusion_divides(cuda, dx):
+    """Quotients by a spacing that is no power of two, within and beyond the range of the two-double reciprocal."""
+    lib = native.load()
+    lib.f2c_diffusion7_v1.argtypes = [c.POINTER(native.Grid), c.c_void_p, c.c_void_p, c.c_double, c.c_double,
+                                      c.c_void_p]
+    a = np.random.default_rng(8).random((42, 52, 72)) * 2.0 ** np.random.default_rng(9).integers(-6, 6, (42, 52, 72))
+    dev = cuda.from_numpy(a).cuda()
+    out = cuda.zeros_like(dev)
+    grid = native.make_grid(70, 50, 40, 1, dx, dx, dx)
+    native.check(lib.f2c_diffusion7_v1(c.byref(grid), dev.data_ptr(), out.data_ptr(), 0.1 * dx * dx, 1.0, None))
+    cuda.cuda.synchronize()
+    ref = np.zeros_like(a)
+    api.diffusion7(ref, a, 0.1 * dx * dx, 1.0, dx, 1)
+    assert np.array_equal(_bits(out.cpu().numpy()), _bits(ref))
+
+
 @pytest.mark.parametrize("how", ["all", "south", "column", "constant"])
 @pytest.mark.parametrize("n", [(31, 1), (65, 33), (2000, 700)])
 def test_planes(cuda, how, n):
