@@ -61,6 +61,10 @@ constexpr int kFaceThreads = kFaceTX * (kFaceTY + 1);
 // registers across the barrier. 512 x 512 x 128 with three scalars: 6.40 ms, at
 // two CTAs 6.41; without scalars 4.13 and 4.44.
 constexpr int kFaceCtasPerSM = 3;
+// One component with at most a scalar needs fewer registers: four CTAs of 56. CDW alone at 512 x 512 x 128 1.47 -> 1.43
+// ms, CDU at 448 x 194 x 26 111 -> 105 us, V with a scalar at 358 x 294 x 88 690 -> 661 us.
+template <int NS, int MASK>
+constexpr int face_ctas_per_sm() { return NS <= 1 && (MASK == 1 || MASK == 2 || MASK == 4) ? 4 : kFaceCtasPerSM; }
 
 // Exact x * 0.5 without the FP64 pipe: for normal x the exponent field drops by
 // one; for the smallest normals and subnormals the significand shifts right
@@ -412,7 +416,7 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
 }
 
 template <int NS, int MASK>
-__global__ void __launch_bounds__(kFaceThreads, kFaceCtasPerSM) advection_faces_kernel(const AdvArgs a) {
+__global__ void __launch_bounds__(kFaceThreads, face_ctas_per_sm<NS, MASK>()) advection_faces_kernel(const AdvArgs a) {
     extern __shared__ double smem[];
     const int k0 = blockIdx.z * a.kz;
     faces_tile<NS, MASK>(a, blockIdx.x, blockIdx.y, k0, min(k0 + a.kz, a.nz), smem);
