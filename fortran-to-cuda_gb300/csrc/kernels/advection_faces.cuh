@@ -87,11 +87,15 @@ __device__ __forceinline__ double exact_half(double x) {
 // `-x`, or a sign flip written in C++, becomes a floating negation that the
 // compiler issues on the FP64 pipe here (measured: three FP64 additions per
 // point fewer, 2 % faster, results unchanged).
+#ifdef __CUDA_ARCH__
 __device__ __forceinline__ double opaque_negate(double x) {
     unsigned long long r;
     asm("xor.b64 %0, %1, 0x8000000000000000;" : "=l"(r) : "l"((unsigned long long)__double_as_longlong(x)));
     return __longlong_as_double((long long)r);
 }
+#else
+__device__ __forceinline__ double opaque_negate(double x) { return -x; }
+#endif
 
 // Whether the high word is zero but for the sign (zero, or far below what the integer products take).
 __device__ __forceinline__ bool zero_high(double x) { return ((unsigned)__double2hiint(x) << 1) == 0; }
@@ -102,11 +106,15 @@ constexpr int kRestW = 1, kRest = 2;
 // A read-only global load the compiler must issue where it stands (not merged
 // with an earlier load of the same address), so that a value loaded before the
 // tile's barrier need not stay in a register across it.
+#ifdef __CUDA_ARCH__
 __device__ __forceinline__ double ldg_again(const double *q) {
     double v;
     asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(q));
     return v;
 }
+#else
+__device__ __forceinline__ double ldg_again(const double *q) { return *q; }
+#endif
 
 template <int NS, int MASK>
 struct FaceSmem {
@@ -415,12 +423,14 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
 #undef LD
 }
 
+#ifdef __CUDACC__
 template <int NS, int MASK>
 __global__ void __launch_bounds__(kFaceThreads, face_ctas_per_sm<NS, MASK>()) advection_faces_kernel(const AdvArgs a) {
     extern __shared__ double smem[];
     const int k0 = blockIdx.z * a.kz;
     faces_tile<NS, MASK>(a, blockIdx.x, blockIdx.y, k0, min(k0 + a.kz, a.nz), smem);
 }
+#endif
 
 // Depth of the z-chunks of one launch: the one with the least time on the SM
 // with the most CTAs, whose levels (and about half a level for a chunk's start)
@@ -444,6 +454,7 @@ inline int chunk_depth(int nx, int ny, int nz) {
     return depth;
 }
 
+#ifdef __CUDACC__
 template <int NS, int MASK>
 cudaError_t launch_faces(const AdvArgs &a, cudaStream_t stream) {
     using Smem = FaceSmem<NS, MASK>;
@@ -458,5 +469,6 @@ cudaError_t launch_faces(const AdvArgs &a, cudaStream_t stream) {
     advection_faces_kernel<NS, MASK><<<grid, block, Smem::bytes, stream>>>(b);
     return cudaGetLastError();
 }
+#endif
 
 } // namespace f2c

@@ -149,6 +149,7 @@ static __device__ __noinline__ void fast_point_fp64(const AdvArgs &a, int i, int
     }
 }
 
+#ifdef __CUDA_ARCH__
 // An 8-byte copy from global to shared memory that runs on while the thread does (cp.async).
 __device__ __forceinline__ void fetch(long long *to, const double *from) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
@@ -156,6 +157,12 @@ __device__ __forceinline__ void fetch(long long *to, const double *from) {
 __device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+#else
+__device__ __forceinline__ void fetch(long long *to, const double *from) { *to = __double_as_longlong(*from); }
+__device__ __forceinline__ void fetch_commit() {}
+template <int N>
+__device__ __forceinline__ void fetch_wait() {}
+#endif
 
 // One tile: columns [tile_x*32, +32) x [tile_y*TY, +TY) of the interior, levels
 // [k0, k1), for one output mode (ADVANCE: forward Euler, else the tendency).
@@ -396,6 +403,7 @@ __device__ __forceinline__ void fast_tile(const AdvArgs &a, int tile_x, int tile
     }
 }
 
+#ifdef __CUDACC__
 template <int NS, int MASK, int TY, int CTAS = fast_ctas_per_sm<TY>()>
 __global__ void __launch_bounds__(fast_threads<TY>(), CTAS)
     advection_fast_kernel(const __grid_constant__ AdvArgs a) {
@@ -403,6 +411,7 @@ __global__ void __launch_bounds__(fast_threads<TY>(), CTAS)
     const int k0 = blockIdx.z * a.kz;
     fast_tile<NS, MASK, TY>(a, blockIdx.x, blockIdx.y, k0, min(k0 + a.kz, a.nz), wide_smem);
 }
+#endif
 
 // z-chunk depth of one launch: the one that takes the fewest level-times, waves
 // of CTAs times the levels of a chunk and its start (two levels unpacked before
@@ -425,6 +434,7 @@ inline int fast_chunk_depth(int nx, int ny, int nz, int ty, int sms) {
     return depth;
 }
 
+#ifdef __CUDACC__
 template <int NS, int MASK, int TY>
 cudaError_t launch_fast(const AdvArgs &a, int sms, cudaStream_t stream) {
     using Sm = FastSmem<NS, TY>;
@@ -439,5 +449,6 @@ cudaError_t launch_fast(const AdvArgs &a, int sms, cudaStream_t stream) {
     kernel<<<grid, block, Sm::bytes, stream>>>(b);
     return cudaGetLastError();
 }
+#endif
 
 } // namespace f2c

@@ -108,6 +108,7 @@ __device__ __forceinline__ void store_point_t(double *out, const double *in, lon
     }
 }
 
+#ifdef __CUDACC__
 // Direct z-marching kernel: one thread per (i, j) column of a BX x BY tile,
 // marching KZ levels. Every value is read through the read-only path; the
 // per-point expressions are those of advection_point.cuh.
@@ -211,5 +212,6 @@ inline cudaError_t launch_halo(const HaloArgs &a, cudaStream_t stream) {
     halo_fill_kernel<<<dim3((unsigned)rows, (unsigned)a.count, 1), dim3(threads, 1, 1), 0, stream>>>(a);
     return cudaGetLastError();
 }
+#endif
 
 } // namespace f2c

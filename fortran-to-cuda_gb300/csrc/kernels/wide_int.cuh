@@ -52,18 +52,13 @@ __device__ __forceinline__ Wide wide_pack(double x, int n) {
     return r;
 }
 
+#ifdef __CUDA_ARCH__
 // m >> n for any n >= 0 (the PTX shift stops at the width).
 __device__ __forceinline__ long long wide_shift(long long m, int n) {
     long long r;
     asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(m), "r"(n));
     return r;
 }
-
-// The significand at the exponent top - headroom: top is the largest exponent of the stencil plus the headroom.
-__device__ __forceinline__ long long wide_align(Wide a, int top) { return wide_shift(a.m, top - a.e); }
-
-__device__ __forceinline__ int max3(int a, int b, int c) { return __vimax3_s32(a, b, c); }
-
 // The words of a significand as 32-bit integers: the high one, and the low one's
 // upper 29 bits. Inline PTX, so that the compiler sees plain 32-bit operands and
 // multiplies them by the one-instruction 32 x 32 + 64 form; from shifts it knows
@@ -85,6 +80,24 @@ __device__ __forceinline__ long long wide_twice(long long m) {
     asm("add.s64 %0, %1, %1;" : "=l"(r) : "l"(m));
     return r;
 }
+// T rounded to 53 bits.
+__device__ __forceinline__ double wide_convert(long long T) {
+    double t;
+    asm("cvt.rn.f64.s64 %0, %1;" : "=d"(t) : "l"(T));
+    return t;
+}
+#else
+__device__ __forceinline__ long long wide_shift(long long m, int n) { return m >> (n < 63 ? n : 63); }
+__device__ __forceinline__ int wide_high(long long m) { return (int)(m >> 32); }
+__device__ __forceinline__ int wide_low(long long m) { return (int)((unsigned)m >> 3); }
+__device__ __forceinline__ long long wide_twice(long long m) { return m + m; }
+__device__ __forceinline__ double wide_convert(long long T) { return (double)T; }
+#endif
+
+// The significand at the exponent top - headroom: top is the largest exponent of the stencil plus the headroom.
+__device__ __forceinline__ long long wide_align(Wide a, int top) { return wide_shift(a.m, top - a.e); }
+
+__device__ __forceinline__ int max3(int a, int b, int c) { return __vimax3_s32(a, b, c); }
 
 // A sum of products' leading 64 bits.
 struct WideSum {
@@ -132,15 +145,16 @@ __device__ __forceinline__ void wide_scale(Wide &w, long long r) {
 // `ke` is that field less one. The conversion rounds T to 53 bits, the product
 // (or multiply-add) rounds once more. Where the factor is below the normal range
 // the product is taken 2^512 larger first (the results there are subnormal or
-// zero); above it `fits` is cleared.
+// zero); above it `fits` is cleared, whatever T is: the exponent of an infinity
+// or NaN lands there with an ordinary significand, and a T of zero (a flow at
+// rest, faces that cancel) says nothing about its product with one.
 template <bool ADD>
 __device__ __forceinline__ double wide_result(long long T, int e, int khi, int klo, int ke, double old, bool &fits) {
-    double t;
-    asm("cvt.rn.f64.s64 %0, %1;" : "=d"(t) : "l"(T));
+    double t = wide_convert(T);
     fits = true;
     double factor = __hiloint2double(khi + (e << 20), klo);
     if ((unsigned)(e + ke) >= 2046u) {
-        if (e + ke >= 2046) fits = T == 0;
+        if (e + ke >= 2046) fits = false;
         if (e + ke < -500 || T == 0) {
             factor = 0.0;
         } else {
