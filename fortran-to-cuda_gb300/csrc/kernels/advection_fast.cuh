@@ -251,7 +251,7 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
         else put_level_as(from, to, std::false_type{});
     };
     // levels k0-1 (slot 2: own column, and W's frame) and k0 (slot 0); level k0+1 on its way
-    Wide wem{0, 0}, wnm{0, 0};
+    Wide wem{0, 0}, wnm{0, 0};  // W east and north of the column a level down (U and V read them): carried up
     fetch_level(ahead, p - plane, plane);
     fetch_level(ahead + Sm::AHEAD, p, plane);
     fetch_wait<1>();
@@ -309,7 +309,7 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
             // (pu, pv, pw: over the component's own part of it)
             const int pu = max3(max3(u0.e, uw.e, up.e), max3(un.e, ue.e, us.e), um.e), EU = max3(pu, uwn.e, uwp.e);
             const int pv = max3(max3(v0.e, vs.e, vp.e), max3(vn.e, ve.e, vw.e), vm.e), EV = max3(pv, ves.e, vsp.e);
-            const int pw = max3(max3(w0.e, wm.e, wp.e), max3(wn.e, we.e, ww.e), ws.e), EW = max3(pw, wem.e, wnm.e);
+            const int pw = max3(max3(w0.e, wm.e, wp.e), max3(wn.e, we.e, ww.e), ws.e), EW = DU || DV ? max3(pw, wem.e, wnm.e) : pw;
             const int E = max3(EU, EV, EW);
             const int du = E - EU, dv = E - EV, dw = E - EW;
             const int tu = EU + 3, tv = EV + 3, tw = EW + 3;
@@ -357,8 +357,10 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
                 const long long T = wide_component(awp, awm, awe, aww, awn, aws, aw0, dw, q, qw, du, r, rs, dv);
                 finish(2, T, EW + E, pw + max3(max3(wp.e, wm.e, u0.e), max3(up.e, uw.e, uwp.e), max(max3(v0.e, vp.e, vs.e), vsp.e)));
             }
-            wem = we;
-            wnm = wn;
+            if (DU || DV) {
+                wem = we;
+                wnm = wn;
+            }
             if (NS > 0) {
                 const int faces = max(max3(u0.e, uw.e, v0.e), max3(vs.e, w0.e, wm.e));
                 const long long east = wide_shift(au0, du), west = -wide_shift(auw, du), north = wide_shift(av0, dv),
