@@ -22,18 +22,24 @@
 // reference (0.5/d along the component, 0.125/d across) are exactly 2A and A/2,
 // and Un-Us = n-s, so the flux and advective forms share every sum. V and W
 // rotate the roles (compiler/tests/fixtures/stencils/{cvd,cdw}.f90:61-66,
-// 89-94). With every velocity in units of its direction's coefficient over x's,
-// the three directions of a component, and a scalar's six faces
-// (advection_point.cuh), are one sum of products times one coefficient.
+// 89-94). A component is the sum over the directions, each in units of its
+// coefficient over x's, times one coefficient; so is a scalar with its six faces
+// (advection_point.cuh).
 //
 // Precision: a field's values at a point's stencil keep 60 bits below the
-// largest of them (an FP64 operation 53 below its own operands), so that a
-// result is off by its two final roundings and 2^-56 or so of (largest
-// component value) x (largest velocity) in the stencil, whatever the tile.
-// Against extended precision the errors (2-norm and maximum) are 0.5 of the FP64
-// form's over the fields of the workloads, equal at worst. What the integers
-// cannot take (infinities, NaN, a value beside the point's own factors that is
-// far larger than they are) goes to FP64 point by point.
+// largest of them (an FP64 operation 53 below its own operands). Each direction
+// is summed at the scale of its own factors, and brought to the largest of the
+// three: along the component that is its difference's scale (a nearly uniform
+// wind's is small), across it the crossing velocity's. A result is off by its two
+// final roundings and 2^-56 or so of that, whatever the tile. Summed at one
+// scale, the largest velocity's, a wind of 10 lost a digit for each factor of ten
+// between it and a cross flow below 1e-2 (1.7e-11 of the maximum at 1e-6; the
+// FP64 form 2e-16). Against exact sums the errors (2-norm) are 0.1 to 1.1 of the
+// FP64 form's over the workloads' fields, uniform and nearly uniform winds,
+// jets, vortices and random exponents, but where both are at the two final
+// roundings (1.5e-16). What the integers cannot take (infinities, NaN, a value
+// beside the point's own factors that is far larger than they are) goes to FP64
+// point by point.
 //
 // Each value is unpacked once, by the thread that owns its cell (the frame's by
 // the threads in turn), and read by its neighbours from shared memory. Values
@@ -86,7 +92,7 @@ constexpr int fast_threads() { return kFastTX * TY; }
 template <int TY>
 constexpr int fast_ctas_per_sm() { return TY <= 4 ? 4 : (TY <= 8 ? 2 : 1); }
 
-// Exponents above a field's own factors' at which it still keeps more bits than FP64: 60 - 5 of them.
+// Exponents above the values that a component reads itself at which it still keeps as many bits as FP64: 60 - 5 of them.
 constexpr int kWideSlack = 5;
 
 constexpr int kFastTY = 8;  // tile height of the single-instance launches
@@ -169,7 +175,7 @@ __device__ __forceinline__ void fetch_wait() {}
 // Called by every thread of a (32, TY) block; `smem` holds
 // FastSmem<NS, TY>::bytes. Starts with the buffers free; a caller that goes on to
 // another tile has a barrier in between.
-template <int NS, int MASK, int TY, bool ADVANCE>
+template <int NS, int MASK, int TY, bool ADVANCE, bool SCALED>
 __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int tile_y, int k0, int k1,
                                                long long *smem) {
     constexpr bool DU = MASK & 1, DV = (MASK >> 1) & 1, DW = (MASK >> 2) & 1;
@@ -189,9 +195,8 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
     long long *const ahead = smem + 3 * LEVEL + warp * kFastTX + lane;  // this thread's values on their way
     short *const ring_e = reinterpret_cast<short *>(smem + 3 * LEVEL + 2 * Sm::AHEAD);
     auto field = [&](int f) { return f == 0 ? a.u : (f == 1 ? a.v : (f == 2 ? a.w : a.s[f - 3])); };
-    auto put = [&](int at, int f, double x, auto scaled) {
-        Wide w = wide_pack(x, f < 3 ? c.wide_shift[f] : 0);
-        if (decltype(scaled)::value && (f == 1 || f == 2)) wide_scale(w, c.wide_ratio[f]);
+    auto put = [&](int at, double x) {
+        const Wide w = wide_pack(x);
         ring[at] = w.m;
         ring_e[at] = (short)w.e;
     };
@@ -200,7 +205,7 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
     // north-west and V south-east): one value of one field to each of the first FIELDS * FRAME turns of the threads.
     constexpr int TURNS = Sm::TURNS;
     const double *frame_at[TURNS];
-    int frame_to[TURNS], frame_field[TURNS];
+    int frame_to[TURNS];
 #pragma unroll
     for (int t = 0; t < TURNS; ++t) {
         const int n = t * kFastTX * TY + warp * kFastTX + lane;
@@ -215,7 +220,6 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
             if (f == g) base = field(g);
         frame_at[t] = base + (i0 + col + a.h) + sx * (long long)(j0 + row + a.h) + plane * (long long)(k0 - 1 + a.h);
         frame_to[t] = use ? f * PLANE + (row + 1) * PITCH + col + 1 : -1;
-        frame_field[t] = f;
     }
     const int own = (warp + 1) * PITCH + lane + 1;
     const long long p0 = (long long)(i + a.h) + sx * (long long)(j + a.h) + plane * (long long)(k0 + a.h);
@@ -235,20 +239,15 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
         }
         fetch_commit();
     };
-    auto put_level_as = [&](const long long *from, int to, auto scaled) {
+    auto put_level = [&](const long long *from, int to) {
         if (inside) {
 #pragma unroll
-            for (int f = 0; f < FIELDS; ++f) put(to + f * PLANE + own, f, __longlong_as_double(from[f * Sm::THREADS]), scaled);
+            for (int f = 0; f < FIELDS; ++f) put(to + f * PLANE + own, __longlong_as_double(from[f * Sm::THREADS]));
         }
 #pragma unroll
         for (int t = 0; t < TURNS; ++t) {
-            if (frame_to[t] >= 0)
-                put(to + frame_to[t], frame_field[t], __longlong_as_double(from[(FIELDS + t) * Sm::THREADS]), scaled);
+            if (frame_to[t] >= 0) put(to + frame_to[t], __longlong_as_double(from[(FIELDS + t) * Sm::THREADS]));
         }
-    };
-    auto put_level = [&](const long long *from, int to) {
-        if (c.wide_scaled) put_level_as(from, to, std::true_type{});
-        else put_level_as(from, to, std::false_type{});
     };
     // levels k0-1 (slot 2: own column, and W's frame) and k0 (slot 0); level k0+1 on its way
     Wide wem{0, 0}, wnm{0, 0};  // W east and north of the column a level down (U and V read them): carried up
@@ -295,6 +294,21 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
                 return Wide{next[n], next_e[n]};
             };
             auto under = [&](int f) { return Wide{prev[f * PLANE], prev_e[f * PLANE]}; };
+            unsigned slow = 0;  // the fields to be done again in FP64
+            // whether the new value has ghost images (store_filled), or is a W wall face
+            const bool images = filled && (across || k < a.h || k >= a.nz - 1 - a.h);
+            // a component's or scalar's value from its sum T at exponent e, stored
+            auto finish = [&](int f, long long T, int e) {
+                const int g = f < 3 ? 0 : 1;
+                double *o = f < 3 ? a.out[f] : a.st[f - 3];
+                bool fits;
+                const double t = wide_result<ADVANCE>(T, e, c.wide_hi[g], c.wide_lo[g], c.wide_e[g],
+                                                      ADVANCE ? old[ADVANCE ? f : 0] : 0.0, fits);
+                if (!fits) slow |= 1u << f;
+                if (!o) return;
+                if (images) store_filled(o, f == 2 ? 1 : 0, a, i, j, k, t);
+                else o[p] = t;
+            };
             const Wide z{0, 0};
             // the stencil of U, V and W, each field aligned to its own largest exponent in it
             const Wide u0 = at(0, 0, 0), v0 = at(1, 0, 0), w0 = at(2, 0, 0);
@@ -306,12 +320,10 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
             const Wide ves = DU ? at(1, -1, 1) : z, vsp = DW ? over(1, -1, 0) : z;
             const Wide wm = under(2), we = DU || DV || DW ? at(2, 0, 1) : z, wn = DU || DV || DW ? at(2, 1, 0) : z;
             const Wide ww = DW ? at(2, 0, -1) : z, ws = DW ? at(2, -1, 0) : z, wp = DW ? over(2, 0, 0) : z;
-            // (pu, pv, pw: over the component's own part of it)
+            // (pu, pv, pw: over what the component reads of itself)
             const int pu = max3(max3(u0.e, uw.e, up.e), max3(un.e, ue.e, us.e), um.e), EU = max3(pu, uwn.e, uwp.e);
             const int pv = max3(max3(v0.e, vs.e, vp.e), max3(vn.e, ve.e, vw.e), vm.e), EV = max3(pv, ves.e, vsp.e);
             const int pw = max3(max3(w0.e, wm.e, wp.e), max3(wn.e, we.e, ww.e), ws.e), EW = DU || DV ? max3(pw, wem.e, wnm.e) : pw;
-            const int E = max3(EU, EV, EW);
-            const int du = E - EU, dv = E - EV, dw = E - EW;
             const int tu = EU + 3, tv = EV + 3, tw = EW + 3;
             const long long au0 = wide_align(u0, tu), auw = wide_align(uw, tu), aun = wide_align(un, tu),
                             aup = wide_align(up, tu);
@@ -319,52 +331,66 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
                             avp = wide_align(vp, tv);
             const long long aw0 = wide_align(w0, tw), awm = wide_align(wm, tw), awe = wide_align(we, tw),
                             awn = wide_align(wn, tw);
-            // a component's or scalar's value from its sum T at exponent e, stored; `slow` notes what does not fit,
-            // and what is computed at a scale above 2^kWideSlack times its own largest factors' (`used`): next to a
-            // value much larger than the ones that it reads itself
-            unsigned slow = 0;
-            // whether the new value has ghost images (store_filled), or is a W wall face
-            const bool images = filled && (across || k < a.h || k >= a.nz - 1 - a.h);
-            auto finish = [&](int f, long long T, int e, int used) {
-                const int g = f < 3 ? f : 3;
-                double *o = f < 3 ? a.out[f] : a.st[f - 3];
-                bool fits;
-                const double t = wide_result<ADVANCE>(T, e, c.wide_hi[g], c.wide_lo[g], c.wide_e[g],
-                                                      ADVANCE ? old[ADVANCE ? f : 0] : 0.0, fits);
-                if (!fits || e - used > kWideSlack) slow |= 1u << f;
-                if (!o) return;
-                if (images) store_filled(o, f == 2 ? 1 : 0, a, i, j, k, t);
-                else o[p] = t;
+            // the fields' exponents against the least of what a component reads of them: a point next to a value much
+            // larger than those (one test for the three components; one a component cost 3 %)
+            const int ux = max(u0.e, uw.e), vx = max(v0.e, vs.e), wx = max(w0.e, wm.e), far = 1 << 14;
+            const int lu = min(DU ? pu : far, min(DV ? max3(ux, un.e, uwn.e) : far, DW ? max3(ux, up.e, uwp.e) : far));
+            const int lv = min(DV ? pv : far, min(DU ? max3(vx, ve.e, ves.e) : far, DW ? max3(vx, vp.e, vsp.e) : far));
+            const int lw = min(DW ? pw : far, min(DU ? max3(wx, we.e, wem.e) : far, DV ? max3(wx, wn.e, wnm.e) : far));
+            if (max3(EU - lu, EV - lv, EW - lw) > kWideSlack) slow |= 7u;
+            // a component P's three sums brought to the largest of their scales: along its own axis (A, lifted by n bits)
+            // and across the two others; FP, F2 and F3 are the exponents of P and of the velocities across, in units of
+            // the directions' coefficients over x's
+            auto component = [&](int f, WideLifted A, long long B2, long long B3, int EP, int FP, int F2, int F3) {
+                const int F1 = FP - A.n, FX = max(F2, F3), F = max(F1, FX);
+                // (a difference not lifted whole, with less across: too few bits)
+                if (A.n == kWideLiftMost - 1 && F1 > FX) slow |= 1u << f;
+                A.m = wide_shift(A.m, F - F1);
+                B2 = wide_shift(B2, F - F2);
+                B3 = wide_shift(B3, F - F3);
+                long long T;
+                if (SCALED) {  // x's sum is the one that is not multiplied
+                    T = f == 0 ? A.m + wide_scaled_sum(B2, c.wide_ratio[1], B3, c.wide_ratio[2])
+                               : B2 + wide_scaled_sum(A.m, c.wide_ratio[f], B3, c.wide_ratio[3 - f]);
+                } else {
+                    T = A.m + B2 + B3;
+                }
+                finish(f, T, EP + F);
             };
+            const int hv = c.wide_shift[1], hw = c.wide_shift[2], FU = EU, FV = EV + hv, FW = EW + hw;
             if (DU) {
                 const long long aue = wide_align(ue, tu), aus = wide_align(us, tu), aum = wide_align(um, tu);
                 const long long q = av0 + ave, qs = avs + wide_align(ves, tv);
                 const long long r = aw0 + awe, rb = awm + wide_align(wem, tw);
-                const long long T = wide_component(aue, auw, aun, aus, aup, aum, au0, du, q, qs, dv, r, rb, dw);
-                finish(0, T, EU + E, pu + max3(max3(ue.e, uw.e, v0.e), max3(ve.e, vs.e, ves.e), max(max3(w0.e, we.e, wm.e), wem.e)));
+                component(0, wide_along(aue, auw, au0), wide_across(aun, aus, au0, q, qs),
+                          wide_across(aup, aum, au0, r, rb), EU, FU, FV, FW);
             }
             if (DV) {
                 const long long avn = wide_align(vn, tv), avw = wide_align(vw, tv), avm = wide_align(vm, tv);
                 const long long q = au0 + aun, qw = auw + wide_align(uwn, tu);
                 const long long r = aw0 + awn, rb = awm + wide_align(wnm, tw);
-                const long long T = wide_component(avn, avs, ave, avw, avp, avm, av0, dv, q, qw, du, r, rb, dw);
-                finish(1, T, EV + E, pv + max3(max3(vn.e, vs.e, u0.e), max3(un.e, uw.e, uwn.e), max(max3(w0.e, wn.e, wm.e), wnm.e)));
+                component(1, wide_along(avn, avs, av0), wide_across(ave, avw, av0, q, qw),
+                          wide_across(avp, avm, av0, r, rb), EV, FV, FU, FW);
             }
             if (DW) {
                 const long long awp = wide_align(wp, tw), aww = wide_align(ww, tw), aws = wide_align(ws, tw);
                 const long long q = au0 + aup, qw = auw + wide_align(uwp, tu);
                 const long long r = av0 + avp, rs = avs + wide_align(vsp, tv);
-                const long long T = wide_component(awp, awm, awe, aww, awn, aws, aw0, dw, q, qw, du, r, rs, dv);
-                finish(2, T, EW + E, pw + max3(max3(wp.e, wm.e, u0.e), max3(up.e, uw.e, uwp.e), max(max3(v0.e, vp.e, vs.e), vsp.e)));
+                component(2, wide_along(awp, awm, aw0), wide_across(awe, aww, aw0, q, qw),
+                          wide_across(awn, aws, aw0, r, rs), EW, FW, FU, FV);
             }
             if (DU || DV) {
                 wem = we;
                 wnm = wn;
             }
             if (NS > 0) {
-                const int faces = max(max3(u0.e, uw.e, v0.e), max3(vs.e, w0.e, wm.e));
-                const long long east = wide_shift(au0, du), west = -wide_shift(auw, du), north = wide_shift(av0, dv),
-                                south = -wide_shift(avs, dv), top = wide_shift(aw0, dw), bottom = -wide_shift(awm, dw);
+                // the six faces' velocities at their own largest exponent, in units of the directions' coefficients over x's
+                const int E = max3(max(u0.e, uw.e), max(v0.e, vs.e) + hv, max(w0.e, wm.e) + hw);
+                const int tu = E + 1, tv = E + (SCALED ? 0 : 1) - hv, tw = E + (SCALED ? 0 : 1) - hw;  // (scaled: halved)
+                auto scaled = [&](long long m, int n) { return SCALED ? wide_scale(m, c.wide_ratio[n]) : m; };
+                const long long east = wide_shift(u0.m, tu - u0.e), west = -wide_shift(uw.m, tu - uw.e);
+                const long long north = wide_shift(scaled(v0.m, 1), tv - v0.e), south = -wide_shift(scaled(vs.m, 1), tv - vs.e);
+                const long long top = wide_shift(scaled(w0.m, 2), tw - w0.e), bottom = -wide_shift(scaled(wm.m, 2), tw - wm.e);
 #pragma unroll
                 for (int n = 0; n < NS; ++n) {
                     const Wide s0 = at(3 + n, 0, 0), se = at(3 + n, 0, 1), sw = at(3 + n, 0, -1), sn = at(3 + n, 1, 0),
@@ -378,10 +404,10 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
                     sum.add(south, wide_align(ss, ts) + as0);
                     sum.add(top, wide_align(sp, ts) + as0);
                     sum.add(bottom, wide_align(sm, ts) + as0);
-                    finish(3 + n, sum.value(), ES + E, ES + faces);
+                    finish(3 + n, sum.value(), ES + E);
                 }
             }
-            if (E >= c.wide_limit) slow = ~0u;
+            if (max3(EU, EV, EW) >= c.wide_limit) slow = ~0u;
             if (slow) fast_point_fp64<filled, ADVANCE>(a, i, j, k, slow);
         }
         below = slot;
@@ -389,19 +415,24 @@ __device__ __forceinline__ void fast_tile_mode(const AdvArgs &a, int tile_x, int
     }
 }
 
-// The tile in the instance's output mode. The mode is a template argument of
-// the tile so that a tendency's first term of each sum is a plain product
-// (pmul, off the FP64 pipe) rather than an FMA with a zero addend, which a
-// runtime choice would leave on the FP64 pipe; a filled advance is an advance.
+// The tile in the instance's output mode and spacing, both template arguments
+// of the loop over the levels: an advance asks for the old values ahead of their
+// use and ends in a multiply-add (a filled advance is an advance), and spacings
+// whose ratios are no powers of two multiply the directions' sums (a branch at
+// each of them instead cost 10 % with either spacing).
 template <int NS, int MASK, int TY>
 __device__ __forceinline__ void fast_tile(const AdvArgs &a, int tile_x, int tile_y, int k0, int k1,
                                           long long *smem) {
+    auto tile = [&](auto advance) {
+        if (a.f.wide_scaled) fast_tile_mode<NS, MASK, TY, decltype(advance)::value, true>(a, tile_x, tile_y, k0, k1, smem);
+        else fast_tile_mode<NS, MASK, TY, decltype(advance)::value, false>(a, tile_x, tile_y, k0, k1, smem);
+    };
     if constexpr ((MASK & kFillMask) != 0) {
-        fast_tile_mode<NS, MASK, TY, true>(a, tile_x, tile_y, k0, k1, smem);
+        tile(std::true_type{});
     } else if (a.mode != 0) {
-        fast_tile_mode<NS, MASK, TY, true>(a, tile_x, tile_y, k0, k1, smem);
+        tile(std::true_type{});
     } else {
-        fast_tile_mode<NS, MASK, TY, false>(a, tile_x, tile_y, k0, k1, smem);
+        tile(std::false_type{});
     }
 }
 

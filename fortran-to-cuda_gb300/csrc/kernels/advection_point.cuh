@@ -108,15 +108,15 @@ struct FastCoefficients {
     double gx, gy, gz;    // diagonal: -0.125/d (times dt)
     double cx, cy, cz;    // cross: -0.0625/d (times dt)
     double sx, sy, sz;    // scalar: 0.5/d (times dt)
-    // Its evaluation in 64-bit fixed point (wide_int.cuh): every velocity in units
-    // of its direction's coefficient over x's (1, dx/dy, dx/dz), so that a
-    // component, and a scalar, is one sum of products times one coefficient.
-    long long wide_ratio[3];     // that ratio's significand in [1/2, 1) times 2^62, a multiple of 8 (wide_scale)
-    int wide_shift[3];           // its exponent (wide_pack), one less where no significand is multiplied
-    int wide_scaled;             // a ratio is not a power of two: V and W are multiplied
+    // Its evaluation in 64-bit fixed point (wide_int.cuh): a component, and a
+    // scalar, is the sum over the directions of the direction's coefficient over
+    // x's (1, dx/dy, dx/dz) times its products, times one coefficient.
+    long long wide_ratio[3];     // that ratio's significand in [1/2, 1) times 2^63 (wide_scale)
+    int wide_shift[3];           // its exponent, one less where no significand is multiplied
+    int wide_scaled;             // a ratio is not a power of two: the y and z sums are multiplied
     int wide_limit;              // exponents from here on are left to FP64 (0: all, a coefficient is out of range)
-    int wide_hi[4], wide_lo[4];  // the coefficients' words (U, V, W, scalars) and their
-    int wide_e[4];               // exponent fields less one, the sums' constants taken off (wide_result)
+    int wide_hi[2], wide_lo[2];  // the coefficients' words (components, scalars) and their
+    int wide_e[2];               // exponent fields less one, the sums' constants taken off (wide_result)
 };
 
 inline FastCoefficients make_fast_coefficients(double dx, double dy, double dz, int advance, double dt) {
@@ -125,32 +125,32 @@ inline FastCoefficients make_fast_coefficients(double dx, double dy, double dz, 
     f.gx = -(0.125 / dx) * t; f.gy = -(0.125 / dy) * t; f.gz = -(0.125 / dz) * t;
     f.cx = -(0.0625 / dx) * t; f.cy = -(0.0625 / dy) * t; f.cz = -(0.0625 / dz) * t;
     f.sx = (0.5 / dx) * t; f.sy = (0.5 / dy) * t; f.sz = (0.5 / dz) * t;
-    // ratio[n] + rest[n] is d0/d to twice a double's precision, inverse[n] its reciprocal rounded once
-    const double d[3] = {dx, dy, dz};
     f.wide_scaled = 0;
     f.wide_limit = 4096;
-    for (int n = 0; n < 4; ++n) {
-        const double ratio = n < 3 ? dx / d[n] : 1.0, inverse = n < 3 ? d[n] / dx : 1.0;
-        // the component's coefficient c0 / ratio, the scalars' -s0
-        const double k = n < 3 ? f.cx * inverse + f.cx * (std::fma(-inverse, dx, d[n]) / dx) : -f.sx;
-        int e = 0, ke = 0;
-        std::frexp(k, &ke);
-        if (!std::isfinite(k) || k == 0.0 || ke < -900 || ke > 900) f.wide_limit = 0;
+    for (int n = 0; n < 2; ++n) {
+        const double k = n == 0 ? f.cx : -f.sx;
+        int e = 0;
+        std::frexp(k, &e);
+        if (!std::isfinite(k) || k == 0.0 || e < -900 || e > 900) f.wide_limit = 0;
         uint64_t bits;
         std::memcpy(&bits, &k, sizeof bits);
-        const int offset = n < 3 ? 2100 : 2101;  // of 2^(e + e') in a sum of products (wide_result)
+        const int offset = n == 0 ? 2100 : 2103;  // of 2^(e + e') in a sum of products (wide_result)
         f.wide_e[n] = (int)((bits >> 52) & 0x7ff) - offset - 1;
         f.wide_hi[n] = (int)((uint32_t)(bits >> 32) - ((uint32_t)offset << 20));
         f.wide_lo[n] = (int)(uint32_t)bits;
-        if (n < 3) {
-            const double m = std::frexp(ratio, &e), rest = std::ldexp(std::fma(-ratio, d[n], dx) / d[n], -e);
-            if (!(ratio > 0.0) || !std::isfinite(ratio) || e < -900 || e > 900) f.wide_limit = 0;
-            f.wide_ratio[n] = f.wide_limit ? (((long long)std::ldexp(m, 62) + (long long)std::ldexp(rest, 62)) & ~7LL) : 0;
-            f.wide_shift[n] = e - 1;
-            if (m != 0.5 || rest != 0.0) f.wide_scaled = 1;
-        }
     }
-    if (f.wide_scaled) {  // V and W are multiplied by a significand below one
+    const double d[3] = {dx, dy, dz};
+    for (int n = 0; n < 3; ++n) {
+        // m 2^e + rest is dx/d to twice a double's precision
+        int e = 0;
+        const double ratio = dx / d[n];
+        const double m = std::frexp(ratio, &e), rest = std::ldexp(std::fma(-ratio, d[n], dx) / d[n], -e);
+        if (!(ratio > 0.0) || !std::isfinite(ratio) || e < -900 || e > 900) f.wide_limit = 0;
+        f.wide_ratio[n] = f.wide_limit ? (long long)std::ldexp(m, 63) + (long long)std::ldexp(rest, 63) : 0;
+        f.wide_shift[n] = e - 1;
+        if (m != 0.5 || rest != 0.0) f.wide_scaled = 1;
+    }
+    if (f.wide_scaled) {  // the y and z sums are multiplied by a significand below one
         ++f.wide_shift[1];
         ++f.wide_shift[2];
     }

@@ -11,15 +11,17 @@
 // No rounding depends on the order of the terms, or on which tile has the point.
 //
 // Ranges. An unpacked |m| is below 2^63, aligned with a headroom of h bits below
-// 2^(63-h). With h = 3: two values' sum or difference is below 2^61, the sums of
-// four below 2^62, f1 + f0 + 4c below 6 x 2^60; a product's high words stay
-// below 2^60.6 and its middle ones (the low word's upper 29 bits) below 2^60.4,
-// so that a component's five products add up below 2^62.7 in both. A scalar's
-// values have h = 2, its velocities 3: six products of 2^58, middle words of 2^59.
+// 2^(63-h). A component's values and the velocities across have h = 3: two
+// values' sum or difference is below 2^61, the sums of four below 2^62, f1 + f0 +
+// 4c below 6 x 2^60, and a difference is lifted to below 2^62; a direction's
+// products add up below 2^61 in the high words and in the middle ones (the low
+// word's upper 29 bits), the three directions below 2^62.6. A scalar's values
+// have h = 2, its velocities 1: six products of 2^60, middle words of 2^60.
 // Dropped: the value bits beyond the alignment's 60 (61), three bits of each low
-// word and the low words' product, together at most 27 and about one unit of
-// 2^-56 times (power of two above the largest component value) times (that of
-// the largest velocity).
+// word, the low words' product, and the directions' bits below the largest one's
+// lowest, together at most 27 and about one unit of 2^-56 times (power of two
+// above the largest component value) times (that of the largest velocity across
+// or of the difference along).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -29,21 +31,21 @@ constexpr int kWideSpecial = 8192;  // the exponent of infinities and NaN
 
 struct Wide {
     long long m;  // signed significand: 53 bits from bit 62 down
-    int e;        // biased exponent (of the value times 2^n, see wide_pack)
+    int e;        // biased exponent
 };
 
-// x * 2^n: a negative significand one's complemented (2^-62 of it off), zero and
+// A negative significand one's complemented (2^-62 of it off), zero and
 // subnormals without the leading bit, infinities and NaN as kWideSpecial.
-__device__ __forceinline__ Wide wide_pack(double x, int n) {
+__device__ __forceinline__ Wide wide_pack(double x) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const int e = (int)((hi >> 20) & 0x7ffu);
     const long long s = (long long)((int)hi >> 31);
     Wide r;
-    r.e = e + n;
+    r.e = e;
     r.m = (long long)((((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo) << 10) ^ s;
     if ((unsigned)(e - 1) >= 2046u) {
         if (e == 0) {
-            r.e = 1 + n;
+            r.e = 1;
             r.m = (long long)((((unsigned long long)(hi & 0xfffffu) << 32) | lo) << 10) ^ s;
         } else {
             r.e = kWideSpecial;
@@ -80,6 +82,12 @@ __device__ __forceinline__ long long wide_twice(long long m) {
     asm("add.s64 %0, %1, %1;" : "=l"(r) : "l"(m));
     return r;
 }
+// The left shift that would bring the high word's leading bit that is not a sign to bit 31 (2^32 - 1: there is none).
+__device__ __forceinline__ unsigned wide_lead(long long m) {
+    unsigned r;
+    asm("bfind.shiftamt.s32 %0, %1;" : "=r"(r) : "r"(wide_high(m)));
+    return r;
+}
 // T rounded to 53 bits.
 __device__ __forceinline__ double wide_convert(long long T) {
     double t;
@@ -91,6 +99,7 @@ __device__ __forceinline__ long long wide_shift(long long m, int n) { return m >
 __device__ __forceinline__ int wide_high(long long m) { return (int)(m >> 32); }
 __device__ __forceinline__ int wide_low(long long m) { return (int)((unsigned)m >> 3); }
 __device__ __forceinline__ long long wide_twice(long long m) { return m + m; }
+__device__ __forceinline__ unsigned wide_lead(long long m) { const int h = wide_high(m) ^ (wide_high(m) >> 31); return h ? (unsigned)__builtin_clz((unsigned)h) : ~0u; }
 __device__ __forceinline__ double wide_convert(long long T) { return (double)T; }
 #endif
 
@@ -112,32 +121,53 @@ struct WideSum {
     __device__ __forceinline__ long long value() const { return high + (middle >> 29); }
 };
 
-// A momentum component's sum: f1, f0 and c along it (one cell either side, and
-// the point), a1, a0 and b1, b0 across its two other axes, q, qn (r, rn) the
-// crossing velocity's face sums at the two faces of that axis, each shifted by
-// its field's distance from the largest exponent:
-//   2[(f1-f0)(f1+f0+4c) + (a1-a0)(q+qn) + (b1-b0)(r+rn)] + (a1+a0+2c)(q-qn) + (b1+b0+2c)(r-rn).
-__device__ __forceinline__ long long wide_component(long long f1, long long f0, long long a1, long long a0, long long b1,
-                                                    long long b0, long long c, int d, long long q, long long qn, int dq,
-                                                    long long r, long long rn, int dr) {
+constexpr int kWideLiftMost = 29;    // of a difference whose high word is all sign, or next to it
+constexpr int kWideNone = 1 << 13;   // a zero's lift: below every other scale
+
+// A product times 2^(n + 1).
+struct WideLifted {
+    long long m;
+    int n;
+};
+
+// A momentum component along its own axis, half its products' sum, with the
+// component one cell either side and at the point:
+//   (f1 - f0)(f1 + f0 + 4c),
+// the difference lifted by n + 1 bits, to below 2^62 and, but for one whose high
+// word is all sign, above 2^61: in a nearly uniform flow it is what is small.
+// (Lifting by the 64 bits' leading one spilled registers: 512 x 512 x 128 with
+// three scalars 1.75 ms instead of 1.56. The caller has FP64 for what the high
+// word does not lift whole.)
+__device__ __forceinline__ WideLifted wide_along(long long f1, long long f0, long long c) {
     WideSum s;
-    const long long c2 = wide_twice(c);
-    s.add(wide_shift(f1 - f0, d), (f1 + f0) + wide_twice(c2));
-    s.add(a1 - a0, wide_shift(q + qn, dq));
-    s.add(b1 - b0, wide_shift(r + rn, dr));
-    s.high = wide_twice(s.high);
-    s.middle = wide_twice(s.middle);
-    s.add((a1 + a0) + c2, wide_shift(q - qn, dq));
-    s.add((b1 + b0) + c2, wide_shift(r - rn, dr));
+    const long long d = f1 - f0;
+    const int lift = (int)min(wide_lead(d) - 2u, (unsigned)kWideLiftMost);
+    s.add(d << lift, (f1 + f0) + wide_twice(wide_twice(c)));
+    return {s.value(), d == 0 ? kWideNone : lift - 1};
+}
+
+// A momentum component across another axis: a1, a0 and c one cell either side of
+// the point and there, q, qn the crossing velocity's face sums on the two sides:
+//   2(a1 - a0)(q + qn) + (a1 + a0 + 2c)(q - qn).
+__device__ __forceinline__ long long wide_across(long long a1, long long a0, long long c, long long q, long long qn) {
+    WideSum s;
+    s.add(wide_twice(a1 - a0), q + qn);
+    s.add((a1 + a0) + wide_twice(c), q - qn);
     return s.value();
 }
 
-// A packed value times a ratio in (1/2, 1) given as `r` = ratio * 2^62, a
-// multiple of 8 (so that the sum's dropped bits are zero): 2^-59 of it off.
-__device__ __forceinline__ void wide_scale(Wide &w, long long r) {
+// m times a significand r in [1/2, 1) (given as 2^63 r), halved.
+__device__ __forceinline__ long long wide_scale(long long m, long long r) {
     WideSum s;
-    s.add(w.m, r);
-    w.m = s.value() << 2;
+    s.add(m, r);
+    return s.value();
+}
+// a times r plus b times t, for |a|, |b| below 2^62 (doubled, for the bits that a product drops).
+__device__ __forceinline__ long long wide_scaled_sum(long long a, long long r, long long b, long long t) {
+    WideSum s;
+    s.add(wide_twice(a), r);
+    s.add(wide_twice(b), t);
+    return s.value();
 }
 
 // T * 2^e * k (plus `old` where ADD), for the coefficient k whose words are

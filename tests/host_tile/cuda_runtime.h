@@ -67,6 +67,7 @@ inline double __dadd_rn(double a, double b) { return a + b; }
 inline double __dmul_rn(double a, double b) { return a * b; }
 inline double __fma_rn(double a, double b, double c) { return std::fma(a, b, c); }
 inline int __clzll(long long x) { return x == 0 ? 64 : __builtin_clzll((unsigned long long)x); }
+inline long long __mul64hi(long long a, long long b) { return (long long)(((__int128)a * b) >> 64); }
 inline int __vimax3_s32(int a, int b, int c) { return max(max(a, b), c); }
 
 using cudaError_t = int;
