@@ -145,6 +145,23 @@ __device__ __forceinline__ double add_rn_range(double a, double b, SumRange &ran
     return __longlong_as_double((long long)(r + ((unsigned long long)((xh & 0xFFF00000u) + ((unsigned)(top - 62) << 20)) << 32)));
 }
 
+// A product that mul_rn_range left, done again: of a zero (fields at rest and
+// plateaus are made of them) on the integer pipes as well, others in FP64.
+__device__ __forceinline__ bool is_zero(double x) {
+    const unsigned long long i = (unsigned long long)__double_as_longlong(x);
+    return ((high_word(i) << 1) | low_word(i)) == 0;
+}
+__device__ __forceinline__ bool is_finite(double x) {
+    return (high_word((unsigned long long)__double_as_longlong(x)) & 0x7FF00000u) != 0x7FF00000u;
+}
+__device__ __forceinline__ double mul_rn_left(double a, double b) {
+    if ((is_zero(a) && is_finite(b)) || (is_zero(b) && is_finite(a)))
+        return __longlong_as_double((__double_as_longlong(a) ^ __double_as_longlong(b)) & (long long)0x8000000000000000ULL);
+    return mul_rn_hw(a, b);
+}
+// Out of line, for kernels whose common path would otherwise make room for it.
+static __device__ __noinline__ double mul_rn_again(double a, double b) { return mul_rn_left(a, b); }
+
 // The same with operands outside the range going to the hardware operation.
 __device__ __forceinline__ double add_rn_int(double a, double b) {
     SumRange range;

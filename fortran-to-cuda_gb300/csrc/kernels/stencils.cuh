@@ -26,8 +26,11 @@
 // A diffusion warp that sees a zero among the values its integer operations
 // would read (a region at rest, an outer row) goes to FP64 at once instead of
 // doing the point twice: 256^3 of zeros 0.48 -> 0.33 ms with dx 1, 1.63 -> 0.33
-// with dx 0.3. In the Yee kernels the same choice cost fields without zeros more
-// (0.238 -> 0.249 ms at 4096^2) than it gave those of zeros (107 -> 99 us at 2048^2).
+// with dx 0.3. In the Yee kernels the same choice costs fields without zeros more
+// (0.238 -> 0.249 ms at 4096^2); there a point done again leaves products of zeros
+// to the integers (mul_rn_again). 4096^2 at rest: 0.37-0.38 ms with every sum in
+// FP64, 0.40-0.41 with FP64 products in the points done again, 0.32 now; fields of
+// plateaus, whose points mix both, 0.31-0.33, 0.40-0.41 and 0.37.
 namespace f2c {
 
 // x * 2^e for an exact power-of-two factor, on the integer pipe when the
@@ -207,8 +210,8 @@ static __global__ void __launch_bounds__(kYeeBX *kYeeBY) yee_h_kernel(const YeeA
         double x = hx - mul_rn_range(p.ch, add_rn_range(north, sign_flipped(e), sums), range);
         double y = hy + mul_rn_range(p.ch, east - e, range);
         if (range.left() || sums.left()) {
-            x = hx - mul_rn_hw(p.ch, north - e);
-            y = hy + mul_rn_hw(p.ch, east - e);
+            x = hx - mul_rn_again(p.ch, north - e);
+            y = hy + mul_rn_again(p.ch, east - e);
         }
         p.hx[q] = x;
         p.hy[q] = y;
@@ -230,7 +233,7 @@ static __global__ void __launch_bounds__(kYeeBX *kYeeBY) yee_e_kernel(const YeeA
         ProductRange<false> range;
         SumRange sums;
         double e = ez + mul_rn_range(p.ce, (hy - west) - add_rn_range(hx, sign_flipped(south), sums), range);
-        if (range.left() || sums.left()) e = ez + mul_rn_hw(p.ce, (hy - west) - (hx - south));
+        if (range.left() || sums.left()) e = ez + mul_rn_again(p.ce, (hy - west) - (hx - south));
         p.ez[q] = e;
         south = hx;
     }

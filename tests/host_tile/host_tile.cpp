@@ -9,6 +9,7 @@
 
 #include "advection_fast.cuh"
 #include "advection_faces.cuh"
+#include "../soft_fp64/operations.h"
 
 namespace {
 using namespace f2c;
@@ -100,4 +101,13 @@ extern "C" void host_fp64_form(const double *const *in, double *const *out, int 
                 if (mode) fast_point_fp64<false, true>(a, i, j, k, ~0u);
                 else fast_point_fp64<false, false>(a, i, j, k, ~0u);
             }
+}
+
+// An operation of tests/soft_fp64/operations.h on n pairs.
+extern "C" void host_operations(int op, const double *a, const double *b, double *out, unsigned char *left, long long n) {
+    for (long long i = 0; i < n; ++i) {
+        bool l;
+        out[i] = soft_cases::operation(op, a[i], b[i], l);
+        left[i] = l;
+    }
 }
