@@ -159,6 +159,16 @@ __device__ __forceinline__ double mul_rn_left(double a, double b) {
         return __longlong_as_double((__double_as_longlong(a) ^ __double_as_longlong(b)) & (long long)0x8000000000000000ULL);
     return mul_rn_hw(a, b);
 }
+// A sum that add_rn_range left, done again in the same way: with a zero, and of opposite numbers.
+__device__ __forceinline__ double add_rn_left(double a, double b) {
+    const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
+    if (is_finite(a) && is_finite(b)) {
+        if (is_zero(a)) return is_zero(b) ? __longlong_as_double(ia & ib) : b;
+        if (is_zero(b)) return a;
+        if ((ia ^ ib) == (long long)0x8000000000000000ULL) return 0.0;
+    }
+    return add_rn_hw(a, b);
+}
 // Out of line, for kernels whose common path would otherwise make room for it.
 static __device__ __noinline__ double mul_rn_again(double a, double b) { return mul_rn_left(a, b); }
 

@@ -46,6 +46,7 @@ __device__ __forceinline__ double scale_pow2(double x, int e, double factor) {
     const int ex = (int)((unsigned long long)b >> 52) & 0x7ff;
     const int r = ex + e;
     if (ex != 0 && ex != 0x7ff && r >= 1 && r <= 0x7fe) return __longlong_as_double(b + ((long long)e << 52));
+    if (((unsigned long long)b << 1) == 0) return x;  // (the factor is 2^e)
     return scale_by(x, factor);
 }
 
@@ -160,7 +161,8 @@ struct JacobiArgs {
 constexpr int kJacBX = 64, kJacBY = 4, kJacJY = 8;  // most rows a thread does
 
 // 8192^2: 0.27 ms with one of the three additions on the integer pipes (0.39 with
-// none, 0.34 with three in two rows).
+// none, 0.34 with three in two rows). At rest 0.39 (0.54 with every sum in FP64
+// or with a zero's sums and scaling done again there).
 static __global__ void __launch_bounds__(kJacBX *kJacBY) jacobi5_kernel(const JacobiArgs p) {
     const int i = blockIdx.x * kJacBX + threadIdx.x;
     const int j0 = (blockIdx.y * kJacBY + threadIdx.y) * p.rows;
@@ -176,7 +178,7 @@ static __global__ void __launch_bounds__(kJacBX *kJacBY) jacobi5_kernel(const Ja
         SumRange sums;
         const double across = west + east;
         double three = add_rn_range(across, south, sums);
-        if (sums.left()) three = add_rn_hw(across, south);
+        if (sums.left()) three = add_rn_left(across, south);
         p.v[q] = scale_pow2(three + north, -2, 0.25);
         south = centre;
         centre = north;

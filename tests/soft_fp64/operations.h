@@ -24,6 +24,6 @@ __device__ __forceinline__ double operation(int op, double a, double b, bool &le
         left = range.left();
         return r;
     }
-    return f2c::mul_rn_again(a, b);
+    return op == 3 ? f2c::mul_rn_again(a, b) : f2c::add_rn_left(a, b);
 }
 }  // namespace soft_cases

@@ -12,7 +12,7 @@ import pytest
 import host_tile
 from test_soft_fp64 import HERE, KERNELS
 
-OPERATIONS = {"product": 0, "wide product": 1, "sum": 2, "product again": 3}
+OPERATIONS = {"product": 0, "wide product": 1, "sum": 2, "product again": 3, "sum again": 4}
 SPECIAL = [0.0, 5e-324, 1e-310, 2.0**-1022, 2.0**-959, 2.0**-512, 2.0**-511, 0.1, 0.75, 1.0, 1.0 + 2.0**-52, 1.5, 3.0,
            2.0**53 - 1, 2.0**511, 2.0**512, 2.0**944, 2.0**945, 1e300, np.finfo(float).max, np.inf, np.nan]
 
@@ -34,7 +34,7 @@ def _exponent(x):
 
 def _check(op, a, b, got, left):
     with np.errstate(all="ignore"):
-        want = a + b if op == 2 else a * b
+        want = a + b if op in (2, 4) else a * b
     ea, eb = _exponent(a), _exponent(b)
     if op == 0:
         may = (ea < 512) | (ea > 1534) | (eb < 512) | (eb > 1534)
