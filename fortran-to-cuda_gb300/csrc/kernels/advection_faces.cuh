@@ -27,7 +27,12 @@
 // again in FP64. A warp that starts a chunk beside zero velocities (a region at
 // rest, a flow without W) takes the products they are in in FP64 from the start:
 // 256 x 256 x 128 with W zero 1.77 -> 1.29 ms, at rest 1.77 -> 1.60 (a choice
-// level by level cost fields without zeros 4 %). Operation count per point: U, V, W: 9 face sums + 18 flux
+// level by level cost fields without zeros 4 %). Products of zeros (a uniform flow
+// has no differences) need no FP64 where the advective half is done again: uniform
+// 512 x 512 x 128 without scalars 5.86 -> 5.01 ms, 100 x 80 x 40 92 -> 82 us (5.81
+// ms and 90 us with 27 products on the integer pipes). So do one component's alone
+// beside zeros: U without V and W, 256 x 256 x 128, 570 -> 513 us (525); with all
+// three that cost fields without zeros 1 %. Operation count per point: U, V, W: 9 face sums + 18 flux
 // products + 15 flux differences + 48 advective-form operations = 90; scalars: 3
 // shared coefficient products + 11 per scalar. Of the 126 with three scalars 69
 // are left to the FP64 pipe. Measured at 512 x 512 x 128 without and with three
@@ -147,6 +152,7 @@ struct FaceSmem {
 template <int NS, int MASK>
 __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int tile_y, int k0, int k1, double *smem) {
     constexpr bool DO_U = MASK & 1, DO_V = MASK & 2, DO_W = MASK & 4, FILL = (MASK & kFillMask) != 0;
+    constexpr bool ONE = MASK == 1 || MASK == 2 || MASK == 4;  // velocity component
     using Smem = FaceSmem<NS, MASK>;
     constexpr int NF = Smem::NF;
     double *xface = smem;                         // [2][NF][XF]
@@ -258,7 +264,7 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
                     FWz = mul(mul(c.Az, sWz), sWz);
                 }
             };
-            auto fp64 = [](double x, double y) { return x * y; };
+            auto fp64 = [](double x, double y) { return ONE ? mul_rn_left(x, y) : x * y; };
             if (REST) fluxes(std::integral_constant<int, 2>{}, fp64);
             if (REST && (rest & kRest)) {
                 fluxes(std::integral_constant<int, 1>{}, fp64);
@@ -391,7 +397,7 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
                     aW[2] = mul(mul(c.Bwz, sub(LDA(W, 0, 0, 1), Wm)), Wc);
                 }
             };
-            auto fp64 = [](double x, double y) { return x * y; };
+            auto fp64 = [](double x, double y) { return ONE ? mul_rn_left(x, y) : x * y; };
             auto difference = [](double x, double y) { return x - y; };
             if (REST) advective(std::integral_constant<int, 2>{}, fp64, difference);
             if (REST && (rest & kRest)) {
@@ -403,7 +409,7 @@ __device__ __forceinline__ void faces_tile(const AdvArgs &a, int tile_x, int til
                 advective(which, [&](double x, double y) { return mul_rn_range(x, y, range); },
                           [&](double x, double y) { return add_rn_range(x, opaque_negate(y), sums); });
                 if (range.left() || sums.left())
-                    advective(which, [](double x, double y) { return mul_rn_hw(x, y); }, difference);
+                    advective(which, [](double x, double y) { return mul_rn_again(x, y); }, difference);
             }
             if (DO_U) {
                 const double r = opaque_negate(((xf[0 * Smem::XF + xo] - xf[0 * Smem::XF + xw]) + (yf[0 * Smem::YF + yo] - yf[0 * Smem::YF + ys])) + (FUz - FUzb));
