@@ -82,10 +82,21 @@ __device__ __forceinline__ long long wide_twice(long long m) {
     asm("add.s64 %0, %1, %1;" : "=l"(r) : "l"(m));
     return r;
 }
-// The left shift that would bring the high word's leading bit that is not a sign to bit 31 (2^32 - 1: there is none).
-__device__ __forceinline__ unsigned wide_lead(long long m) {
-    unsigned r;
-    asm("bfind.shiftamt.s32 %0, %1;" : "=r"(r) : "r"(wide_high(m)));
+// The left shift that brings the leading bit of d that is not a sign, below bit
+// 61, to bit 61; above every exponent where there is none (a zero has no scale).
+// A search in each word: the 64-bit one cost registers, which the step spilled
+// (512 x 512 x 128 with three scalars 1.75 ms instead of 1.53).
+__device__ __forceinline__ int wide_lift(long long d) {
+    const int h = wide_high(d);
+    unsigned up, low;
+    asm("bfind.shiftamt.s32 %0, %1;" : "=r"(up) : "r"(h));
+    asm("{.reg .b32 t, u; mov.b64 {t, u}, %1; xor.b32 t, t, u; bfind.shiftamt.u32 %0, t;}" : "=r"(low) : "l"(d));
+    return up == ~0u ? (int)(low & 0x1fffu) + 30 : (int)up - 2;
+}
+// m << n for any n >= 0.
+__device__ __forceinline__ long long wide_shift_left(long long m, int n) {
+    long long r;
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(m), "r"(n));
     return r;
 }
 // T rounded to 53 bits.
@@ -99,7 +110,8 @@ __device__ __forceinline__ long long wide_shift(long long m, int n) { return m >
 __device__ __forceinline__ int wide_high(long long m) { return (int)(m >> 32); }
 __device__ __forceinline__ int wide_low(long long m) { return (int)((unsigned)m >> 3); }
 __device__ __forceinline__ long long wide_twice(long long m) { return m + m; }
-__device__ __forceinline__ unsigned wide_lead(long long m) { const int h = wide_high(m) ^ (wide_high(m) >> 31); return h ? (unsigned)__builtin_clz((unsigned)h) : ~0u; }
+__device__ __forceinline__ int wide_lift(long long d) { const long long m = d < 0 ? ~d : d; return m ? __clzll(m) - 2 : 0x1fff + 30; }
+__device__ __forceinline__ long long wide_shift_left(long long m, int n) { return n < 64 ? (long long)((unsigned long long)m << n) : 0; }
 __device__ __forceinline__ double wide_convert(long long T) { return (double)T; }
 #endif
 
@@ -121,9 +133,6 @@ struct WideSum {
     __device__ __forceinline__ long long value() const { return high + (middle >> 29); }
 };
 
-constexpr int kWideLiftMost = 29;    // of a difference whose high word is all sign, or next to it
-constexpr int kWideNone = 1 << 13;   // a zero's lift: below every other scale
-
 // A product times 2^(n + 1).
 struct WideLifted {
     long long m;
@@ -133,17 +142,14 @@ struct WideLifted {
 // A momentum component along its own axis, half its products' sum, with the
 // component one cell either side and at the point:
 //   (f1 - f0)(f1 + f0 + 4c),
-// the difference lifted by n + 1 bits, to below 2^62 and, but for one whose high
-// word is all sign, above 2^61: in a nearly uniform flow it is what is small.
-// (Lifting by the 64 bits' leading one spilled registers: 512 x 512 x 128 with
-// three scalars 1.75 ms instead of 1.56. The caller has FP64 for what the high
-// word does not lift whole.)
+// the difference lifted by n + 1 bits, its leading one to bit 61: in a nearly
+// uniform flow it is what is small.
 __device__ __forceinline__ WideLifted wide_along(long long f1, long long f0, long long c) {
     WideSum s;
     const long long d = f1 - f0;
-    const int lift = (int)min(wide_lead(d) - 2u, (unsigned)kWideLiftMost);
-    s.add(d << lift, (f1 + f0) + wide_twice(wide_twice(c)));
-    return {s.value(), d == 0 ? kWideNone : lift - 1};
+    const int lift = wide_lift(d);
+    s.add(wide_shift_left(d, lift), (f1 + f0) + wide_twice(wide_twice(c)));
+    return {s.value(), lift - 1};
 }
 
 // A momentum component across another axis: a1, a0 and c one cell either side of
