@@ -55,14 +55,13 @@ def algorithmic_bytes_per_point(nscalar: int, mode: str = "tendency") -> int:
 def fp64_ops_per_point(nscalar: int, numerics: str = "strict", mode: str = "tendency") -> int:
     """FP64-pipe instructions per point of each numerical form's expression DAG (every face value computed once).
 
-    What each kernel issues on the FP64 pipe is ``fp64_pipe_ops_per_point``: the fast-fp kernel evaluates its form
-    in 64-bit integers (wide_int.cuh) and issues far fewer.
-    Products on the integer pipes (``mul_rn_int``, rounded exactly as DMUL) and the exact halving (an exponent
-    decrement) are not counted here (``int_pipe_ops_per_point``).
+    With ``int_pipe_ops_per_point`` it adds up to the form's operations, which is what the bench line reports; the
+    split between the two is that of the first kernels, which had 27 products on the integer pipes. What each kernel
+    issues on the FP64 pipe now is ``fp64_pipe_ops_per_point``.
     strict (the reference grouping): U, V, W: 9 face sums, 15 flux differences, 30 advective-form sums and
     differences, and the first product of each of the 9 face fluxes (the second product of each flux and the 18
-    advective-form products run on the integer pipes); scalars: 3 shared coefficient products, and per scalar 8
-    sums and differences and 3 face-flux products.
+    advective-form products are counted as integer operations); scalars: 3 shared coefficient products, and per
+    scalar 8 sums and differences and 3 face-flux products.
     fast (factored FMA form): U, V, W: 6 face sums + 12 per component (3 for the direction along it, 3 for each
     across, 3 to accumulate, of which a tendency's first is a plain product); scalars: 5 for the shared divergence
     term + 7 FMAs per scalar (6 in a tendency).
@@ -83,8 +82,8 @@ def fp64_pipe_ops_per_point(nscalar: int, numerics: str = "strict", mode: str = 
 
 
 def int_pipe_ops_per_point(nscalar: int, numerics: str = "strict", mode: str = "tendency") -> int:
-    """Floating-point operations per point that run on the integer pipes: products, and the strict kernel's exact
-    halving of U, V, W."""
+    """The form's remaining operations: 27 products of the strict one and its exact halving of U, V, W, the factored
+    one's plain products (see ``fp64_ops_per_point``)."""
     tendency = mode == "tendency"
     if numerics == "fast":
         return 9 + 3 * tendency + (3 + tendency * nscalar if nscalar else 0)

@@ -48,9 +48,11 @@
 // 8 warps of 128 registers, two CTAs per SM; with three (80 registers, spills)
 // 512 x 512 x 128 with three scalars took 1.79 ms instead of 1.54, 4-row tiles
 // 2.1, 16-row tiles 2.1 (each with its frame's share of the unpacking).
-// 512 x 512 x 128 with three scalars: 1.54 ms (the FP64 form 3.95); without
-// scalars 0.88; 257 x 193 x 61 with two, advanced: 170 us (475); 64 instances
-// with one scalar in one batched launch: 3.47 ms (9.43).
+// 512 x 512 x 128 with three scalars: 1.55 ms (the FP64 form 3.95); without
+// scalars 0.94; 257 x 193 x 61 with two, advanced: 162 us (475); 64 instances
+// with one scalar in one batched launch: 3.57 ms (9.44; 3.38 with one scale for
+// all directions, which lost digits). Spacings with no power-of-two ratio: 1.71 ms
+// at the first of these.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -65,8 +65,8 @@ __global__ void __launch_bounds__(kFaceThreads, kFaceCtasPerSM)
     }
 }
 
-// The same persistent loop over the fast-fp tile (advection_fast.cuh), tiles of 32 x TY points: TY + 1
-// warps per CTA; small tiles run more CTAs per SM (the register budget at 96 per thread).
+// The same persistent loop over the fast-fp tile (advection_fast.cuh), tiles of 32 x TY points: TY warps
+// per CTA of 128 registers a thread; small tiles run more CTAs per SM (fast_ctas_per_sm).
 
 template <int NS, int MASK, int TY>
 __global__ void __launch_bounds__(fast_threads<TY>(), fast_ctas_per_sm<TY>())

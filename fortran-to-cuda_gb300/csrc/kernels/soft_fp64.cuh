@@ -32,7 +32,7 @@ static __device__ __noinline__ double mul_rn_hw(double a, double b) { return __d
 
 // Words of a 64-bit pattern. On the device they are inline PTX: where the
 // compiler sees a word as a shift of a value whose range it knows, it multiplies
-// 64 x 64 bits instead of 32 x 32 (70 instructions for the product below, not 41).
+// 64 x 64 bits instead of 32 x 32.
 #ifdef __CUDA_ARCH__
 __device__ __forceinline__ unsigned high_word(unsigned long long x) {
     unsigned r;
@@ -172,7 +172,8 @@ __device__ __forceinline__ double add_rn_left(double a, double b) {
 // Out of line, for kernels whose common path would otherwise make room for it.
 static __device__ __noinline__ double mul_rn_again(double a, double b) { return mul_rn_left(a, b); }
 
-// The same with operands outside the range going to the hardware operation.
+// One operation by itself, operands outside the range going to the hardware's (the kernels use the forms above, which
+// leave that to the end of several).
 __device__ __forceinline__ double add_rn_int(double a, double b) {
     SumRange range;
     const double r = add_rn_range(a, b, range);

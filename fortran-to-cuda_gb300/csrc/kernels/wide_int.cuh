@@ -64,7 +64,7 @@ __device__ __forceinline__ long long wide_shift(long long m, int n) {
 // The words of a significand as 32-bit integers: the high one, and the low one's
 // upper 29 bits. Inline PTX, so that the compiler sees plain 32-bit operands and
 // multiplies them by the one-instruction 32 x 32 + 64 form; from shifts it knows
-// the ranges of, it builds 64 x 64 products instead (16 instructions for 5).
+// the ranges of, it builds 64 x 64 products instead.
 __device__ __forceinline__ int wide_high(long long m) {
     int r;
     asm("{.reg .b32 t; mov.b64 {t, %0}, %1;}" : "=r"(r) : "l"(m));

@@ -75,7 +75,9 @@ int f2c_advection_v1(const f2c_grid_v1 *grid, const f2c_fields_v1 *fields, void 
  *   algebraically regrouped form of the same tendencies, evaluated in 64-bit
  *   fixed point at each point's own scale. Results differ from the oracle by
  *   rounding only: every field within 1e-12 of its maximum magnitude (measured
- *   ~1e-15). In F2C_ADVANCE mode the time step is folded into the coefficients.
+ *   ~1e-15), but where the oracle's own fluxes cancel to less (a strong component
+ *   with small noise along itself). In F2C_ADVANCE mode the time step is folded
+ *   into the coefficients.
  */
 enum f2c_kernel_variant { F2C_KERNEL_FACES = 0, F2C_KERNEL_DIRECT = 1, F2C_KERNEL_FAST = 2 };
 int f2c_advection_variant_v1(const f2c_grid_v1 *grid, const f2c_fields_v1 *fields, int variant, void *stream);

@@ -69,8 +69,8 @@ int f2c_batch_prepare_async_v1(const f2c_grid_v1 *grids, const f2c_fields_v1 *fi
 
 /* Tile shapes. The plans above cut every instance into tiles of 32 x 8
  * columns. These entries take the tile height: 4, 8 or 16 rows (one warp per
- * row; 4-row tiles run four CTAs per SM, 8-row two, 16-row
- * one). Tiles of 4 or 16 rows run the fast-fp kernel only; results do not
+ * row; 4-row tiles run four CTAs per SM, three with three or four scalars,
+ * 8-row two, 16-row one). Tiles of 4 or 16 rows run the fast-fp kernel only; results do not
  * depend on the tile shape or the z-chunk depths, bit for bit. `staging` NULL
  * prepares synchronously on `stream` (as f2c_batch_prepare_v1), otherwise as
  * f2c_batch_prepare_async_v1 does. */
